@@ -268,6 +268,319 @@ __global__ void cell_grad_kernel(Geom g, const double *__restrict__ cellp, int n
   dEdL[5] = D[2][1];
 }
 
+// ---------------------------------------------------------------------------
+// Gather by bricks: the grid block of a brick in shared memory.
+//
+// One CTA takes the points of a brick of TX x TY x 32 cells (whole buckets of
+// the cell sort, so the points are TX TY contiguous runs of the sorted order)
+// and copies the brick's grid block with its stencil halo, rows of 40 values
+// from 4 below the brick, to shared memory with cp.async (periodic images row
+// by row).  One thread then takes one point, reads its P^3 values with
+// constant offsets from one address, and no load passes the L1 tag stage,
+// which bounds the thread-per-point kernel above.
+//
+// Shared-memory wavefronts bound it instead (23 M at 1M points, order 6; 61%
+// of the pipe's peak).  32 lanes at unrelated places cost about 3.4
+// wavefronts per load.  All lanes add the same offset for the same tap, so
+// the lanes of a warp are conflict-free on every load when their origins
+// differ modulo 32: the brick's points are ordered by (rank within their
+// origin's class modulo 32, class), which brings it to 2.0.  The order only
+// decides which thread computes a point, never a result, so the ranks may
+// come from shared-memory atomics.  1M points, order 6, 256^3: 183 -> 135 us.
+template <int P, int TX, int TY, int NT_>
+struct TileCfg {
+  static constexpr int NT = NT_;  // threads
+  static constexpr int RX = TX + P - 1, RY = TY + P - 1, PITCH = 40, Z0 = 4;
+  static constexpr int ROWS = RX * RY, CELLROWS = TX * TY;
+  static constexpr int ITEMS = (TX * TY * 4 + NT - 1) / NT < 2 ? 2 : (TX * TY * 4 + NT - 1) / NT;
+  static constexpr int CAP = ITEMS * NT;             // points ordered at a time
+  static constexpr int LEVELS = 64;                  // ranks that get an exact place; later ones follow in any order
+};
+template <int P, int TX, int TY, int NT>
+struct TileSmem {
+  using C = TileCfg<P, TX, TY, NT>;
+  __align__(16) float tile[C::ROWS * C::PITCH];
+  float4 rec[C::CAP];  // fractions of the points in the conflict-free order
+  uint2 list[C::CAP];  // their input index and origin
+  int rowidx[C::ROWS]; // grid row (x K1 + y) of every tile row
+  int start[C::CELLROWS], pref[C::CELLROWS + 1];
+  uint32_t lmask[C::LEVELS];
+  int lbase[C::LEVELS + 1];
+  __align__(16) int hist[32];
+  int wsum[32], extra;
+};
+
+struct TileArgs {
+  Geom g;
+  const int *cs;        // bucket offsets of the cell sort
+  const uint32_t *perm, *key;
+  const float4 *rec;
+  const double *w;
+  const float *grid;
+  double *dx, *phi;
+  int n, nty, nzb;
+  long nb;
+};
+
+// Enqueues the copies of the brick's tile rows in pieces of V values.
+template <int P, int TX, int TY, int NT, int V>
+__device__ __forceinline__ void tile_copy(const TileArgs &A, TileSmem<P, TX, TY, NT> &sm, int z0) {
+  using C = TileCfg<P, TX, TY, NT>;
+  constexpr int PQ = C::PITCH / V;
+  const int K2 = A.g.K2, nq = K2 / V;
+  const int zq0 = imod(z0 - C::Z0, K2) / V;
+  for (int e = threadIdx.x; e < C::ROWS * PQ; e += NT) {
+    const int r = e / PQ, c = e - r * PQ;
+    int zq = zq0 + c;
+    if (zq >= nq) zq = nq >= PQ ? zq - nq : zq % nq;
+    const long src = (long)sm.rowidx[r] * K2 + V * zq;
+    if (!SPME_IN(src, (long)A.g.K0 * A.g.K1 * K2 - (V - 1), CK_GATHER_GRID)) continue;
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(sm.tile + r * C::PITCH + V * c);
+    if (V == 4) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(A.grid + src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(A.grid + src), "n"(4 * V) : "memory");
+  }
+}
+
+template <int P, int TX, int TY, int NT, bool GRAD, bool POT>
+__global__ void __launch_bounds__(NT, 768 / NT) gather_tile_kernel(TileArgs A, Spline S) {
+  using C = TileCfg<P, TX, TY, NT>;
+  extern __shared__ __align__(16) unsigned char gt_smem[];
+  TileSmem<P, TX, TY, NT> &sm = *reinterpret_cast<TileSmem<P, TX, TY, NT> *>(gt_smem);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const Geom &g = A.g;
+  const int tz = (int)(blockIdx.x % (unsigned)A.nzb), bxy = (int)(blockIdx.x / (unsigned)A.nzb);
+  const int x0 = (bxy / A.nty) * TX, y0 = (bxy % A.nty) * TY, z0 = tz * 32;
+  const bool near = g.K0 >= C::RX && g.K1 >= C::RY;
+  for (int r = tid; r < C::ROWS; r += C::NT) {
+    int xi = x0 + r / C::RY + 1 - P / 2, yi = y0 + r % C::RY + 1 - P / 2;
+    if (near) {
+      xi += xi < 0 ? g.K0 : (xi >= g.K0 ? -g.K0 : 0);
+      yi += yi < 0 ? g.K1 : (yi >= g.K1 ? -g.K1 : 0);
+    } else {
+      xi = imod(xi, g.K0);
+      yi = imod(yi, g.K1);
+    }
+    sm.rowidx[r] = xi * g.K1 + yi;
+  }
+  // the brick's points: one run of the sorted order per cell row
+  int cnt = 0;
+  if (tid < C::CELLROWS) {
+    const int gx = x0 + tid / TY, gy = y0 + tid % TY;
+    if (gx < g.K0 && gy < g.K1) {
+      const long b = ((long)gx * g.K1 + gy) * A.nzb + tz;
+      if (SPME_IN(b, A.nb, CK_GATHER_ROW)) {
+        const int s = __ldg(A.cs + b);
+        cnt = __ldg(A.cs + b + 1) - s;
+        sm.start[tid] = s;
+        if (!SPME_IN(s, A.n + 1, CK_GATHER_ROW) || !SPME_IN(cnt, A.n - s + 1, CK_GATHER_ROW)) cnt = 0;
+      }
+    }
+  }
+  int incl = cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  if (lane == 31) sm.wsum[warp] = incl;
+  __syncthreads();
+  int wpre = 0, total = 0;
+#pragma unroll
+  for (int k = 0; k < C::NT / 32; k++) {
+    const int v = sm.wsum[k];
+    wpre += k < warp ? v : 0;
+    total += v;
+  }
+  if (total == 0) return;  // an empty brick
+  if (tid < C::CELLROWS) sm.pref[tid + 1] = wpre + incl;
+  if (tid == 0) sm.pref[0] = 0;
+  // the grid block in the widest pieces that divide a row (then no piece
+  // crosses the periodic boundary)
+  if ((g.K2 & 3) == 0) tile_copy<P, TX, TY, NT, 4>(A, sm, z0);
+  else if ((g.K2 & 1) == 0) tile_copy<P, TX, TY, NT, 2>(A, sm, z0);
+  else tile_copy<P, TX, TY, NT, 1>(A, sm, z0);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int c0 = 0; c0 < total; c0 += C::CAP) {
+    const int m = min(C::CAP, total - c0);
+    if (tid < 32) sm.hist[tid] = 0;
+    if (tid == 32) sm.extra = 0;
+    __syncthreads();
+    int ploc[C::ITEMS], prank[C::ITEMS];
+    uint32_t pa[C::ITEMS];
+    float4 pr[C::ITEMS];
+#pragma unroll
+    for (int it = 0; it < C::ITEMS; it++) {
+      const int t = tid + it * C::NT;
+      prank[it] = -1;
+      if (t < m) {
+        int lo = 0;  // largest row with pref[row] <= c0 + t
+#pragma unroll
+        for (int step = C::CELLROWS / 2; step > 0; step >>= 1)
+          if (sm.pref[lo + step] <= c0 + t) lo += step;
+        const int a = sm.start[lo] + (c0 + t - sm.pref[lo]);
+        if (SPME_IN(a, A.n, CK_GATHER_ATOM)) {
+          const int rx = lo / TY, ry = lo - rx * TY;
+          const int row = sm.rowidx[(rx + P / 2 - 1) * C::RY + ry + P / 2 - 1];
+          pr[it] = __ldg(A.rec + a);
+          pa[it] = __ldg(A.perm + a);
+          if (!SPME_IN(pa[it], A.n, CK_GATHER_ATOM)) pa[it] = 0;
+          int zl = (int)(__ldg(A.key + a) - (uint32_t)row * (uint32_t)g.K2) - z0;
+          if (!SPME_IN(zl, 32, CK_GATHER_KEY)) zl = 0;
+          ploc[it] = (rx * C::RY + ry) * C::PITCH + zl + C::Z0 + 1 - P / 2;
+          prank[it] = atomicAdd(&sm.hist[ploc[it] & 31], 1);
+        }
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {  // places of the ranks: rank r holds the classes with more than r points
+      uint32_t m0 = 0, m1 = 0;
+#pragma unroll
+      for (int c = 0; c < 32; c += 4) {
+        const int4 h = *reinterpret_cast<const int4 *>(sm.hist + c);
+        m0 |= (h.x > lane ? 1u : 0u) << c | (h.y > lane ? 2u : 0u) << c | (h.z > lane ? 4u : 0u) << c |
+              (h.w > lane ? 8u : 0u) << c;
+        m1 |= (h.x > lane + 32 ? 1u : 0u) << c | (h.y > lane + 32 ? 2u : 0u) << c |
+              (h.z > lane + 32 ? 4u : 0u) << c | (h.w > lane + 32 ? 8u : 0u) << c;
+      }
+      int s0 = __popc(m0), s1 = __popc(m1);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u0 = __shfl_up_sync(0xffffffffu, s0, o), u1 = __shfl_up_sync(0xffffffffu, s1, o);
+        if (lane >= o) {
+          s0 += u0;
+          s1 += u1;
+        }
+      }
+      const int tot0 = __shfl_sync(0xffffffffu, s0, 31);
+      sm.lmask[lane] = m0;
+      sm.lmask[lane + 32] = m1;
+      sm.lbase[lane + 1] = s0;
+      sm.lbase[lane + 33] = tot0 + s1;
+      if (lane == 0) sm.lbase[0] = 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < C::ITEMS; it++) {
+      if (prank[it] < 0) continue;
+      const int c = ploc[it] & 31;
+      const int pos = prank[it] < C::LEVELS
+                          ? sm.lbase[prank[it]] + __popc(sm.lmask[prank[it]] & ((1u << c) - 1u))
+                          : sm.lbase[C::LEVELS] + atomicAdd(&sm.extra, 1);
+      if (SPME_IN(pos, C::CAP, CK_GATHER_ATOM)) {
+        sm.list[pos] = make_uint2(pa[it], (uint32_t)ploc[it]);
+        sm.rec[pos] = pr[it];
+      }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    for (int p = tid; p < m; p += C::NT) {
+      const uint2 e = sm.list[p];
+      const float4 u = sm.rec[p];
+      const uint32_t a = e.x;
+      const double qa = GRAD ? __ldg(A.w + a) : 0.0;
+      const float *q = sm.tile + e.y;
+      float wx[P], dwx[P], wy[P], dwy[P], wz[P], dwz[P];
+#pragma unroll
+      for (int i = 0; i < P; i++) {
+        dbspl_eval(S, P, 1.f - u.x, i, wx[i], dwx[i]);
+        dbspl_eval(S, P, 1.f - u.y, i, wy[i], dwy[i]);
+        dbspl_eval(S, P, 1.f - u.z, i, wz[i], dwz[i]);
+      }
+      // the sums of stencil_sum, term by term in the same order
+      float pot = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
+#pragma unroll
+      for (int i = 0; i < P; i++) {
+        float sy = 0.f, dy = 0.f, dz = 0.f;
+#pragma unroll
+        for (int j = 0; j < P; j++) {
+          float sz = 0.f, dzz = 0.f;
+#pragma unroll
+          for (int k = 0; k < P; k++) {
+            const float v = q[(i * C::RY + j) * C::PITCH + k];
+            sz = fmaf(wz[k], v, sz);
+            if (GRAD) dzz = fmaf(dwz[k], v, dzz);
+          }
+          sy = fmaf(wy[j], sz, sy);
+          if (GRAD) {
+            dy = fmaf(dwy[j], sz, dy);
+            dz = fmaf(wy[j], dzz, dz);
+          }
+        }
+        if (POT) pot = fmaf(wx[i], sy, pot);
+        if (GRAD) {
+          gx = fmaf(dwx[i], sy, gx);
+          gy = fmaf(wx[i], dy, gy);
+          gz = fmaf(wx[i], dz, gz);
+        }
+      }
+      const CellConst &cc = *g.cell;
+      if (GRAD) {
+        const double f = -qa * cc.iV;
+        const double G0 = (double)gx * f * g.K0, G1 = (double)gy * f * g.K1,
+                     G2 = (double)gz * f * g.K2;
+        A.dx[3 * (long)a + 0] = cc.iL00 * G0;
+        A.dx[3 * (long)a + 1] = cc.iL10 * G0 + cc.iL11 * G1;
+        A.dx[3 * (long)a + 2] = cc.iL20 * G0 + cc.iL21 * G1 + cc.iL22 * G2;
+      }
+      if (POT) A.phi[a] = (double)pot * cc.iV;
+    }
+    __syncthreads();
+  }
+}
+
+template <int P, int TX, int TY, int NT, bool GRAD, bool POT>
+static void gather_tile_launch(const TileArgs &A, const Spline &S, cudaStream_t st) {
+  const unsigned blocks = (unsigned)(((A.g.K0 + TX - 1) / TX) * (long)A.nty * A.nzb);
+  gather_tile_kernel<P, TX, TY, NT, GRAD, POT><<<blocks, NT, sizeof(TileSmem<P, TX, TY, NT>), st>>>(A, S);
+}
+
+template <int P, int TX, int TY, int NT>
+static void gather_tile_attr() {
+  const int bytes = (int)sizeof(TileSmem<P, TX, TY, NT>);
+  const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  cudaFuncSetAttribute(gather_tile_kernel<P, TX, TY, NT, true, true>, attr, bytes);
+  cudaFuncSetAttribute(gather_tile_kernel<P, TX, TY, NT, true, false>, attr, bytes);
+  cudaFuncSetAttribute(gather_tile_kernel<P, TX, TY, NT, false, true>, attr, bytes);
+}
+
+template <int P, int TX, int TY, int NT>
+static void gather_tile_t(TileArgs A, const Spline &S, cudaStream_t st) {
+  A.nty = (A.g.K1 + TY - 1) / TY;
+  if (A.dx && A.phi) gather_tile_launch<P, TX, TY, NT, true, true>(A, S, st);
+  else if (A.dx) gather_tile_launch<P, TX, TY, NT, true, false>(A, S, st);
+  else gather_tile_launch<P, TX, TY, NT, false, true>(A, S, st);
+}
+
+// The brick shape: 16 x 8 x 32 cells and 256 threads, 3 CTAs per SM.  A
+// smaller brick copies more halo per point and has more unequal classes, a
+// larger one leaves fewer CTAs to overlap their copies (1M points, order 6,
+// 256^3: 137 us; 8 x 8 with 128 threads 143, 16 x 16 with 256 or 384 threads
+// 147 / 145, 16 x 8 with 128 threads 147).
+constexpr int kTileX = 16, kTileY = 8, kTileThreads = 256;
+
+static void gather_tile(const TileArgs &A, const Spline &S, cudaStream_t st) {
+  if (A.g.order == 6) gather_tile_t<6, kTileX, kTileY, kTileThreads>(A, S, st);
+  else gather_tile_t<8, kTileX, kTileY, kTileThreads>(A, S, st);
+}
+
+// The brick kernel needs enough points to repay its set-up (a dozen dependent
+// steps before the first stencil) and enough taps per point to repay its
+// copy.  Thread per point / bricks, us: order 6, 50k points on 72^3 20.5 / 18.5,
+// 100k on 120^3 26.6 / 25.6, 200k on 120^3 39.8 / 30.7, 400k on 192^3 81 / 55,
+// 1M on 256^3 182 / 135; order 8, 50k on 72^3 28.7 / 30.8, 100k on 120^3
+// 50 / 33, 1M on 256^3 352 / 205; order 4, 100k on 96^3 14.3 / 16.4, 1M on
+// 200^3 77.8 / 79.9 (not taken).  Odd rows are copied value by value: 200k
+// points on 150^3 then took 45.1 us against 45.0 (order 6).
+constexpr int kTileMinPoints = 65536, kTileMinPointsOdd = 262144;
+static bool use_tiles(const Geom &g, int n) {
+  return g.order >= 6 && n >= ((g.K2 & 1) ? kTileMinPointsOdd : kTileMinPoints);
+}
+
+void gather_prepare() {
+  gather_tile_attr<6, kTileX, kTileY, kTileThreads>();
+  gather_tile_attr<8, kTileX, kTileY, kTileThreads>();
+}
+
 template <int P, bool SORTED>
 static int gather_p(const Geom &g, const Spline &S, int n, const double *x, const double *w, const float *grid,
                     double *dx, double *phi, double *cellp, const SortedView &sv, cudaStream_t st) {
@@ -303,8 +616,14 @@ static SortedView make_view(const Geom &g, const uint32_t *perm, const uint32_t 
 
 int launch_gather(const Geom &g, const Spline &S, int n, const double *x, const double *w,
                   const float *grid, double *dx, double *phi, cudaStream_t st, const uint32_t *perm,
-                  const uint32_t *keys, const float4 *rec) {
-  if (n <= 0) return 0;
+                  const uint32_t *keys, const float4 *rec, const int *cs) {
+  if (n <= 0 || (!dx && !phi)) return 0;
+  if (cs && use_tiles(g, n)) {
+    gather_tile(TileArgs{g, cs, perm, keys, rec, w, grid, dx, phi, n, 0, (g.K2 + 31) / 32,
+                         sort_buckets(g, kSpreadZShift)},
+                S, st);
+    return 1;
+  }
   if (perm) return gather_any<true>(g, S, n, x, w, grid, dx, phi, nullptr, make_view(g, perm, keys, rec), st);
   return gather_any<false>(g, S, n, x, w, grid, dx, phi, nullptr, SortedView{}, st);
 }

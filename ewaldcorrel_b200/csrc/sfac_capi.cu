@@ -420,6 +420,7 @@ void *sfac_ctor(double L[6], int K[3], int order) {
   make_spline(order, h->spline, h->nodes);
   fft_prepare_kernels();
   spread_prepare();
+  gather_prepare();
   if (const char *e = getenv("SFAC_NO_GRAPH")) h->use_graph = !(e[0] && e[0] != '0');
   if (const char *e = getenv("SFAC_ZY_MODE")) {
     const int v = atoi(e);
@@ -1081,7 +1082,8 @@ static int enqueue_solve(Handle *h, int n, const double *x, const double *w, dou
     k += launch_gather_cell(h->geom, h->spline, n, x, w, h->d_real, dx, phi, h->d_cellp, ev, dEdL, st, perm, skeys,
                             h->sb.rec_sorted);
   else if (n > 0 && (dx || phi))
-    k += launch_gather(h->geom, h->spline, n, x, w, h->d_real, dx, phi, st, perm, skeys, h->sb.rec_sorted);
+    k += launch_gather(h->geom, h->spline, n, x, w, h->d_real, dx, phi, st, perm, skeys, h->sb.rec_sorted,
+                       h->sb.cell_start);
   if (timed) CK(h, cudaEventRecord(h->ev_stage[6], st));
   return k;
 }

@@ -46,7 +46,7 @@ enum CheckSite : unsigned {
   CK_SORT_BUCKET = 0x101, CK_SORT_SCATTER, CK_SORT_FIXUP, CK_SORT_MERGE,
   CK_SPREAD_BUCKET = 0x201, CK_SPREAD_RANGE, CK_SPREAD_ATOM, CK_SPREAD_CASE, CK_SPREAD_ROW,
   CK_SPREAD_GRID,
-  CK_GATHER_ATOM = 0x301, CK_GATHER_KEY, CK_GATHER_GRID,
+  CK_GATHER_ATOM = 0x301, CK_GATHER_KEY, CK_GATHER_GRID, CK_GATHER_ROW,
   CK_FFT_LINE = 0x401, CK_FFT_CONV,
   CK_SERVE_ATOM = 0x501, CK_SERVE_OUT,
   CK_SELFTEST = 0xf01,

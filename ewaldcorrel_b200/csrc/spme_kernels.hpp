@@ -167,7 +167,8 @@ int launch_finish(const double *partials, int nblocks, const CellConst *cell, do
 // launch_cell_sort) -- points are then gathered in cell order.
 int launch_gather(const Geom &g, const Spline &S, int n, const double *x, const double *w,
                   const float *grid, double *dx, double *phi, cudaStream_t st, const uint32_t *perm = nullptr,
-                  const uint32_t *keys = nullptr, const float4 *rec = nullptr);
+                  const uint32_t *keys = nullptr, const float4 *rec = nullptr, const int *cs = nullptr);
+void gather_prepare();  // sets the brick kernels' shared-memory limits once (before any graph capture)
 // Gather + cell adjoint: dE/dL (6 doubles, device) from dE/dx, the virial in ev
 // and the positions; cellp is scratch of gather_cell_words(n) doubles.
 int launch_gather_cell(const Geom &g, const Spline &S, int n, const double *x, const double *w,
