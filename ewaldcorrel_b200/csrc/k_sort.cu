@@ -212,18 +212,20 @@ static int key_passes(long ncell) {
 //
 //   1. key_count_kernel: keys and records (as above); every atom takes an
 //      arrival slot in its bucket with an integer atomic (count[bucket]++).
-//   2. tile_sum_kernel + cell_offsets_kernel: exclusive scan of the
-//      per-bucket counts, in place, into cell_start (cell_start[nb] = n):
-//      the sum of every tile of 2^tshift buckets, then each tile scans its
-//      buckets from the sum of the tiles before it (at most ~2048 tiles).
-//   3. cell_scatter_kernel: every atom goes to cell_start[bucket] + its
-//      arrival slot, with its key; an atom alone in its bucket is final.
-//   4. cell_fixup_kernel: the atoms of each shared bucket are put in
-//      (key, input index) order -- rank = number of the bucket's atoms with a
-//      smaller (key, index) pair -- which is exactly the stable order of the
-//      reference's multimap.  Buckets with more than kBigCell atoms are
-//      listed and merge-sorted by the last CTA to finish (no waiting on other
-//      CTAs).
+//   2. cell_offsets_kernel: exclusive scan of the per-bucket counts, in
+//      place, into cell_start (cell_start[nb] = n): each tile of 2^tshift
+//      buckets scans from the sum of the tiles before it (at most ~2048
+//      tiles, whose sums the first pass takes, or tile_sum_kernel).
+//   3. by slots: the first pass also left every atom's (key, index) in a slot
+//      of its bucket; cell_place_kernel ranks each atom among them -- the
+//      number of the bucket's atoms with a smaller (key, index) pair, which is
+//      exactly the stable order of the reference's multimap -- and writes it
+//      to its final place.  Without slots: cell_scatter_kernel sends every
+//      atom to cell_start[bucket] + its arrival slot (an atom alone in its
+//      bucket is final) and cell_fixup_kernel ranks them there.  A bucket with
+//      more than kBigCell atoms is merge-sorted by one CTA (no waiting on
+//      other CTAs).
+// Up to kSmallAtoms atoms take one launch of one CTA instead.
 // Only integer atomics (counts) are used; the result is the same bits on
 // every run.
 
@@ -247,16 +249,17 @@ long sort_buckets(const Geom &g, int zshift) {
   return (long)g.K0 * g.K1 * nzb;
 }
 
-// Word layout of the bucket-count region (everything before the tile sums is
-// zeroed before every sort):
+// Word layout of the bucket-count region (zeroed before every sort):
 //   [0, nb + 1)            counts, then offsets
-//   [nb + 1, nb + 3)       control: large buckets, finished fix-up CTAs
-//   [nb + 3, 2 nb + 3)     head: atoms of each bucket in its first H - 1 cells
-//   [2 nb + 3, 3 nb + 3)   tail: atoms of each bucket in its last H cells
-//   [3 nb + 3, + T)        tile sums
+//   [nb + 1, 2 nb + 1)     head: atoms of each bucket in its first H - 1 cells
+//   [2 nb + 1, 3 nb + 1)   tail: atoms of each bucket in its last H cells
+//   [3 nb + 1, + T)        tile sums
+//   [3 nb + 1 + T, + nb)   spill (with slots): last atom (+ 1) of each bucket past its slots
 // (head and tail: the spread's halo of an interior brick starts H cells
 // before a bucket boundary and ends H - 1 cells after one, H = order / 2.)
-size_t cell_count_words(long nb) { return (size_t)(3 * nb + 3 + cell_tiles(nb)); }
+size_t cell_count_words(long nb, bool with_slots) {
+  return (size_t)(3 * nb + 1 + cell_tiles(nb) + (with_slots ? nb : 0));
+}
 
 // Bucket of a cell key (see above).
 struct BucketMap {
@@ -279,29 +282,58 @@ static BucketMap bucket_map(const Geom &g, int zshift) {
   return m;
 }
 
-// head/tail (may be null): see the word layout above; ht_h = H.
+// Slots of the buckets (the sort in two passes): slot s < ns of bucket b
+// holds the (key, index) of its s-th arrival; later arrivals form a chain
+// from spill[b] over next[] (index + 1, 0: the end).
+struct Slots {
+  uint2 *at;
+  int ns;
+  uint32_t *spill, *next;
+};
+
+// head/tail (may be null): see the word layout above; ht_h = H.  tsum (may be
+// null): the counts' tile sums, taken with one atomic per tile and CTA.
+constexpr int kCountTiles = 128;
 __global__ void __launch_bounds__(256) key_count_kernel(Geom g, int n, const double *__restrict__ x,
                                                         const double *__restrict__ w, uint32_t *__restrict__ keys,
                                                         uint32_t *__restrict__ slot, float4 *__restrict__ rec,
                                                         uint32_t *__restrict__ count, BucketMap bm,
                                                         uint32_t *__restrict__ head, uint32_t *__restrict__ tail,
-                                                        int ht_h) {
+                                                        int ht_h, Slots sl, uint32_t *__restrict__ tsum, int tshift,
+                                                        int ntiles) {
+  __shared__ uint32_t th[kCountTiles];
+  if (tsum) {
+    if (threadIdx.x < ntiles) th[threadIdx.x] = 0u;
+    __syncthreads();
+  }
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= n) return;
-  const CellConst cc = *g.cell;
-  float4 r;
-  const uint32_t key = cell_key(g, cc, x[3 * a], x[3 * a + 1], x[3 * a + 2], r, (float)w[a]);
-  keys[a] = key;
-  rec[a] = r;
-  uint32_t row, n2;
-  bm.K2d.divmod(key, row, n2);
-  const uint32_t b = row * bm.nzb + (n2 >> bm.zshift);
-  if (!SPME_IN(b, bm.nb, CK_SORT_BUCKET)) return;
-  slot[a] = atomicAdd(&count[b], 1u);
-  if (head) {
-    const int off = (int)(n2 & ((1u << bm.zshift) - 1u));
-    if (off < ht_h - 1) atomicAdd(&head[b], 1u);
-    if (off >= (1 << bm.zshift) - ht_h) atomicAdd(&tail[b], 1u);
+  if (a < n) {
+    const CellConst cc = *g.cell;
+    float4 r;
+    const uint32_t key = cell_key(g, cc, x[3 * a], x[3 * a + 1], x[3 * a + 2], r, (float)w[a]);
+    keys[a] = key;
+    rec[a] = r;
+    uint32_t row, n2;
+    bm.K2d.divmod(key, row, n2);
+    const uint32_t b = row * bm.nzb + (n2 >> bm.zshift);
+    if (SPME_IN(b, bm.nb, CK_SORT_BUCKET)) {
+      const uint32_t s = atomicAdd(&count[b], 1u);
+      slot[a] = s;
+      if (sl.at) {
+        if (s < (uint32_t)sl.ns) sl.at[(size_t)b * sl.ns + s] = make_uint2(key, (uint32_t)a);
+        else sl.next[a] = atomicExch(&sl.spill[b], (uint32_t)a + 1u);
+      }
+      if (head) {
+        const int off = (int)(n2 & ((1u << bm.zshift) - 1u));
+        if (off < ht_h - 1) atomicAdd(&head[b], 1u);
+        if (off >= (1 << bm.zshift) - ht_h) atomicAdd(&tail[b], 1u);
+      }
+      if (tsum) atomicAdd(&th[b >> tshift], 1u);
+    }
+  }
+  if (tsum) {
+    __syncthreads();
+    if (threadIdx.x < ntiles && th[threadIdx.x]) atomicAdd(&tsum[threadIdx.x], th[threadIdx.x]);
   }
 }
 
@@ -353,9 +385,12 @@ __global__ void __launch_bounds__(kScanThreads) tile_sum_kernel(const uint32_t *
 }
 
 // cs[0 .. nscan): per-bucket counts in, exclusive prefix sums out, one CTA
-// per tile; the tile's base is the sum of the earlier tiles' sums.
+// per tile; the tile's base is the sum of the earlier tiles' sums.  done (at
+// a large bucket's offset): the counter of its atoms that arrived in the
+// merge sort's buffers, zeroed here.
 __global__ void __launch_bounds__(kScanThreads) cell_offsets_kernel(uint32_t *__restrict__ cs, long nscan,
-                                                                    int tshift, const uint32_t *__restrict__ tsum) {
+                                                                    int tshift, const uint32_t *__restrict__ tsum,
+                                                                    uint32_t *__restrict__ done) {
   constexpr int NW = kScanThreads / 32;
   __shared__ uint32_t wsum[NW];
   __shared__ uint32_t red[NW];
@@ -393,6 +428,7 @@ __global__ void __launch_bounds__(kScanThreads) cell_offsets_kernel(uint32_t *__
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
       o[k] = e;
+      if (a[k] > (uint32_t)kBigCell) done[e] = 0u;
       e += a[k];
     }
     if (full) {
@@ -475,21 +511,37 @@ __device__ void big_cell_sort(int lo, int c, uint32_t *tkeys, uint32_t *tmp, uin
   __syncthreads();
 }
 
-// ctl[0]: number of listed large buckets, ctl[1]: finished CTAs (both zero on
-// entry; the last CTA resets ctl[1]).  big: listed bucket indices (capacity n).
+// Merge-sorts the large buckets that threads of this CTA hand in (at most one
+// each; found is false elsewhere).  All threads must call.
+__device__ __forceinline__ void sort_big_buckets(bool found, uint32_t b, const int *__restrict__ cs, uint32_t *tkeys,
+                                                 uint32_t *tmp, uint32_t *skeys, uint32_t *perm,
+                                                 const float4 *__restrict__ rec, float4 *__restrict__ rec_sorted) {
+  if (!__syncthreads_or(found)) return;
+  __shared__ uint32_t list[256];
+  __threadfence();  // the other CTAs' atoms of a handed-in bucket
+  list[threadIdx.x] = found ? b : 0xffffffffu;
+  __syncthreads();
+  for (int t = 0; t < (int)blockDim.x; t++) {
+    const uint32_t bb = list[t];
+    if (bb != 0xffffffffu) big_cell_sort(cs[bb], cs[bb + 1] - cs[bb], tkeys, tmp, skeys, perm, rec, rec_sorted);
+  }
+}
+
 __global__ void __launch_bounds__(256) cell_fixup_kernel(int n, const int *__restrict__ cs, BucketMap bm,
                                                          uint32_t *tkeys, uint32_t *tmp, uint32_t *skeys,
                                                          uint32_t *perm, const float4 *__restrict__ rec,
-                                                         float4 *__restrict__ rec_sorted, uint32_t *ctl,
-                                                         uint32_t *big) {
+                                                         float4 *__restrict__ rec_sorted) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  bool found = false;
+  uint32_t b = 0;
   if (i < n) {
-    const uint32_t key = tkeys[i];
-    const uint32_t b = bm(key);
+    // (a merge sort of this atom's large bucket may run already: its keys stay in the bucket)
+    const uint32_t key = *reinterpret_cast<volatile uint32_t *>(tkeys + i);
+    b = bm(key);
     const bool ok = SPME_IN(b, bm.nb, CK_SORT_BUCKET);
     const int lo = ok ? cs[b] : 0, c = ok ? cs[b + 1] - lo : 1;
     if (c > kBigCell) {
-      if (i == lo) big[atomicAdd(&ctl[0], 1u)] = b;
+      found = i == lo;
     } else if (c > 1) {
       const uint32_t a = tmp[i];
       int r = 0;
@@ -501,21 +553,204 @@ __global__ void __launch_bounds__(256) cell_fixup_kernel(int n, const int *__res
       }
     }
   }
-  // the last CTA to finish sorts the listed large buckets
-  __shared__ bool last;
-  __threadfence();
+  sort_big_buckets(found, b, cs, tkeys, tmp, skeys, perm, rec, rec_sorted);
+}
+
+// Second pass of the sort by slots: every atom reads its bucket's (key,
+// index) pairs from the slots (and the chain past them), counts the smaller
+// ones and writes itself to its final place, in one kernel instead of a
+// scatter and a fix-up.  The atoms
+// of a bucket above kBigCell go to tkeys/tmp; the last of them to arrive
+// hands the bucket to its CTA's merge sort.
+__global__ void __launch_bounds__(256) cell_place_kernel(int n, const uint32_t *__restrict__ keys,
+                                                         const uint32_t *__restrict__ slot,
+                                                         const float4 *__restrict__ rec, const int *__restrict__ cs,
+                                                         BucketMap bm, Slots sl, uint32_t *tkeys, uint32_t *tmp,
+                                                         uint32_t *skeys, uint32_t *perm,
+                                                         float4 *__restrict__ rec_sorted, uint32_t *done) {
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  bool found = false;
+  uint32_t b = 0;
+  if (a < n) {
+    const uint32_t key = keys[a];
+    const float4 r = rec[a];
+    b = bm(key);
+    if (SPME_IN(b, bm.nb, CK_SORT_BUCKET)) {
+      const uint2 *at = sl.at + (size_t)b * sl.ns;
+      const int lo = cs[b], c = cs[b + 1] - lo;
+      if (c > kBigCell) {
+        const int s = (int)slot[a];
+        if (SPME_IN(s, c, CK_SORT_SCATTER)) {
+          tkeys[lo + s] = key;
+          tmp[lo + s] = (uint32_t)a;
+          __threadfence();
+          found = atomicAdd(&done[lo], 1u) == (uint32_t)(c - 1);
+        }
+      } else {
+        int rank = 0;
+        if (c > 1) {
+          const int m = min(c, sl.ns);
+          for (int j = 0; j < m; j += 4) {  // ns is a multiple of 4: whole 32-byte reads stay in the bucket's slots
+            const uint4 p = *reinterpret_cast<const uint4 *>(at + j), q = *reinterpret_cast<const uint4 *>(at + j + 2);
+            rank += pair_less(p.x, p.y, key, (uint32_t)a) ? 1 : 0;
+            rank += j + 1 < m && pair_less(p.z, p.w, key, (uint32_t)a) ? 1 : 0;
+            rank += j + 2 < m && pair_less(q.x, q.y, key, (uint32_t)a) ? 1 : 0;
+            rank += j + 3 < m && pair_less(q.z, q.w, key, (uint32_t)a) ? 1 : 0;
+          }
+          if (c > m)
+            for (uint32_t e = sl.spill[b]; e; e = sl.next[e - 1]) {
+              if (!SPME_IN(e - 1, n, CK_SORT_SCATTER)) break;
+              rank += pair_less(keys[e - 1], e - 1, key, (uint32_t)a) ? 1 : 0;
+            }
+        }
+        if (SPME_IN(rank, c, CK_SORT_FIXUP) && SPME_IN(lo + c - 1, n, CK_SORT_FIXUP)) {
+          skeys[lo + rank] = key;
+          perm[lo + rank] = (uint32_t)a;
+          rec_sorted[lo + rank] = r;
+        }
+      }
+    }
+  }
+  sort_big_buckets(found, b, cs, tkeys, tmp, skeys, perm, rec, rec_sorted);
+}
+
+// The whole sort in one CTA, for few atoms on few buckets: counts, offsets
+// and the (key, index) pairs stay in shared memory, so that the five
+// dependent launches (a memset and four kernels of a few us of latency each)
+// become one.  Same outputs as the passes below.  One SM computes all the
+// FP64 keys, so it pays only while every thread has one atom: solves of 64
+// atoms on 24^3 39 -> 35 us, 1000 on 32^3 44.5 -> 43, but 2048 on 32^3 45.2 ->
+// 47.2 (and 4000 on 40^3 49.3 -> 55.5) with two (four) atoms per thread.
+constexpr int kSmallThreads = 1024, kSmallItems = 1, kSmallAtoms = kSmallThreads * kSmallItems;
+constexpr int kSmallBuckets = 8192;
+static size_t small_sort_smem(long nb, bool ht) {
+  return sizeof(uint32_t) * (size_t)((nb + 1) + (ht ? 2 * nb : 0) + 3) + sizeof(uint2) * kSmallAtoms;
+}
+
+__global__ void __launch_bounds__(kSmallThreads) cell_sort_small_kernel(
+    Geom g, int n, const double *__restrict__ x, const double *__restrict__ w, BucketMap bm, int ht_h, int *cs,
+    uint32_t *__restrict__ head, uint32_t *__restrict__ tail, uint32_t *tkeys, uint32_t *tmp, uint32_t *skeys,
+    uint32_t *perm, float4 *rec, float4 *__restrict__ rec_sorted) {
+  extern __shared__ __align__(16) unsigned char small_smem[];
+  __shared__ uint32_t wsum[kSmallThreads / 32];
+  __shared__ int nbig;
+  __shared__ uint32_t blist[kSmallAtoms / kBigCell];
+  uint2 *pairs = reinterpret_cast<uint2 *>(small_smem);
+  uint32_t *cnt = reinterpret_cast<uint32_t *>(pairs + kSmallAtoms);
+  const int nb = (int)bm.nb, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint32_t *hd = cnt + nb + 1, *tl = hd + nb;
+  const int words = nb + 1 + (ht_h ? 2 * nb : 0);
+  for (int i = tid; i < words; i += kSmallThreads) cnt[i] = 0u;
+  if (tid == 0) nbig = 0;
+  const CellConst cc = *g.cell;
+  uint32_t key[kSmallItems], bk[kSmallItems], slot[kSmallItems];
+  float4 r[kSmallItems];
+#pragma unroll
+  for (int it = 0; it < kSmallItems; it++) {
+    const int a = tid + it * kSmallThreads;
+    key[it] = bk[it] = 0u;
+    if (a < n) key[it] = cell_key(g, cc, x[3 * a], x[3 * a + 1], x[3 * a + 2], r[it], (float)w[a]);
+  }
   __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(&ctl[1], 1u) == gridDim.x - 1;
+#pragma unroll
+  for (int it = 0; it < kSmallItems; it++) {
+    const int a = tid + it * kSmallThreads;
+    if (a < n) {
+      uint32_t row, n2;
+      bm.K2d.divmod(key[it], row, n2);
+      uint32_t b = row * bm.nzb + (n2 >> bm.zshift);
+      if (!SPME_IN(b, nb, CK_SORT_BUCKET)) b = 0;
+      bk[it] = b;
+      slot[it] = atomicAdd(&cnt[b], 1u);
+      if (ht_h) {
+        const int off = (int)(n2 & ((1u << bm.zshift) - 1u));
+        if (off < ht_h - 1) atomicAdd(&hd[b], 1u);
+        if (off >= (1 << bm.zshift) - ht_h) atomicAdd(&tl[b], 1u);
+      }
+    }
+  }
   __syncthreads();
-  if (!last) return;
-  __threadfence();
-  const uint32_t nb = *((volatile uint32_t *)&ctl[0]);
-  for (uint32_t k = 0; k < nb; k++) {
-    const uint32_t b = *((volatile uint32_t *)&big[k]);
-    const int lo = cs[b], c = cs[b + 1] - lo;
+  // exclusive scan of the counts, in place; offsets, heads and tails to global memory
+  const int per = (nb + 1 + kSmallThreads - 1) / kSmallThreads;
+  const int i0 = min(tid * per, nb + 1), i1 = min(i0 + per, nb + 1);
+  uint32_t sum = 0;
+  for (int i = i0; i < i1; i++) sum += cnt[i];
+  uint32_t incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  if (lane == 31) wsum[warp] = incl;
+  __syncthreads();
+  uint32_t e = incl - sum;
+  for (int k = 0; k < warp; k++) e += wsum[k];
+  for (int i = i0; i < i1; i++) {
+    const uint32_t c = cnt[i];
+    cnt[i] = e;
+    if (c > (uint32_t)kBigCell) {
+      const int k = atomicAdd(&nbig, 1);
+      if (SPME_IN(k, kSmallAtoms / kBigCell, CK_SORT_MERGE)) blist[k] = (uint32_t)i;
+    }
+    e += c;
+  }
+  __syncthreads();
+  for (int i = tid; i <= nb; i += kSmallThreads) cs[i] = (int)cnt[i];
+  if (ht_h)
+    for (int i = tid; i < nb; i += kSmallThreads) {
+      head[i] = hd[i];
+      tail[i] = tl[i];
+    }
+#pragma unroll
+  for (int it = 0; it < kSmallItems; it++) {
+    const int a = tid + it * kSmallThreads;
+    if (a < n && SPME_IN(cnt[bk[it]] + slot[it], n, CK_SORT_SCATTER))
+      pairs[cnt[bk[it]] + slot[it]] = make_uint2(key[it], (uint32_t)a);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int it = 0; it < kSmallItems; it++) {
+    const int a = tid + it * kSmallThreads;
+    if (a >= n) continue;
+    const int lo = (int)cnt[bk[it]], c = (int)cnt[bk[it] + 1] - lo;
+    if (c > kBigCell) {
+      tkeys[lo + slot[it]] = key[it];
+      tmp[lo + slot[it]] = (uint32_t)a;
+      rec[a] = r[it];
+    } else {
+      int rank = 0;
+      for (int j = lo; j < lo + c; j++) rank += pair_less(pairs[j].x, pairs[j].y, key[it], (uint32_t)a) ? 1 : 0;
+      if (SPME_IN(rank, c, CK_SORT_FIXUP)) {
+        skeys[lo + rank] = key[it];
+        perm[lo + rank] = (uint32_t)a;
+        rec_sorted[lo + rank] = r[it];
+      }
+    }
+  }
+  __syncthreads();
+  for (int k = 0; k < nbig; k++) {
+    const int lo = (int)cnt[blist[k]], c = (int)cnt[blist[k] + 1] - lo;
     big_cell_sort(lo, c, tkeys, tmp, skeys, perm, rec, rec_sorted);
   }
-  if (threadIdx.x == 0) ctl[1] = 0u;
+}
+
+// The sort by slots takes the place of the scatter and fix-up while a bucket
+// holds few enough atoms for its slots (at a mean of half of them less three,
+// 5 of 16, about one bucket in 70,000 spills) and while the slots, written
+// and read in pieces of 32 bytes, stay small in L2: a solve of 98k atoms on
+// 96^3 (3.5 MB of slots) took 71.9 us against 73.8, 200k on 128^3 132.9 / 134.9,
+// 400k on 160^3 (16 MB) 247.9 / 249.2, but 600k on 192^3 (28 MB) 332.6 / 325.9
+// and 1M on 256^3 (67 MB) 605 / 592.
+constexpr double kSlotsMaxBytes = 1 << 24;
+static bool use_slots(const Geom &g, int n, const SortBuffers &b, int zshift) {
+  const double mean = (double)n * (double)(1 << zshift) / ((double)g.K0 * g.K1 * g.K2);
+  return b.slots && 2.0 * mean + 6.0 <= (double)b.nslot &&
+         8.0 * (double)b.nslot * (double)sort_buckets(g, zshift) <= kSlotsMaxBytes;
+}
+
+void sort_prepare() {
+  cudaFuncSetAttribute((const void *)cell_sort_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)small_sort_smem(kSmallBuckets, true));
 }
 
 // Computes keys/fractions, sorts, and builds the per-bucket offsets.
@@ -529,29 +764,42 @@ int launch_cell_sort(const Geom &g, int n, const double *x, const double *w, Sor
   const int tshift = cell_tile_shift(nb);
   const BucketMap bm = bucket_map(g, zshift);
   uint32_t *count = reinterpret_cast<uint32_t *>(b.cell_start);
-  uint32_t *ctl = count + (nb + 1);
-  uint32_t *head = count + (nb + 3), *tail = count + (2 * nb + 3);
-  uint32_t *tsum = count + (3 * nb + 3);
+  uint32_t *head = count + (nb + 1), *tail = count + (2 * nb + 1);
+  uint32_t *tsum = count + (3 * nb + 1), *spill = tsum + ntiles;
   const int ht_h = zshift > 0 ? g.order / 2 : 0;  // head/tail counts for the spread's buckets only
   b.cur = 0;
-  cudaMemsetAsync(count, 0, sizeof(uint32_t) * ((ht_h ? 3 * nb : nb) + 3), st);
+  if (n <= kSmallAtoms && nb <= kSmallBuckets) {
+    cell_sort_small_kernel<<<1, kSmallThreads, small_sort_smem(nb, ht_h > 0), st>>>(
+        g, n, x, w, bm, ht_h, b.cell_start, head, tail, b.tkeys, b.tmp, b.keys[0], b.vals[0], b.rec, b.rec_sorted);
+    return 1;
+  }
+  const bool slots = use_slots(g, n, b, zshift);
+  // tile sums taken while counting, while they are few (more: one pass over the counts)
+  const bool count_tiles = ntiles > 1 && ntiles <= kCountTiles && n > 0;
+  const Slots sl{slots ? b.slots : nullptr, b.nslot, spill, b.next};
+  cudaMemsetAsync(count, 0, sizeof(uint32_t) * (3 * nb + 1 + ntiles + (slots ? nb : 0)), st);
   int launches = 0;
   if (n > 0) {
     key_count_kernel<<<ceil_div(n, 256), 256, 0, st>>>(g, n, x, w, b.keys[1], b.vals[1], b.rec, count, bm,
-                                                       ht_h ? head : nullptr, tail, ht_h);
+                                                       ht_h ? head : nullptr, tail, ht_h, sl,
+                                                       count_tiles ? tsum : nullptr, tshift, (int)ntiles);
     launches++;
   }
-  if (ntiles > 1) {  // one tile (grids up to about 64^3): its scan starts from 0, no tile sums needed
+  if (ntiles > 1 && !count_tiles) {  // one tile (grids up to about 64^3): its scan starts from 0, no tile sums needed
     tile_sum_kernel<<<(unsigned)ntiles, kScanThreads, 0, st>>>(count, nb + 1, tshift, tsum);
     launches++;
   }
-  cell_offsets_kernel<<<(unsigned)ntiles, kScanThreads, 0, st>>>(count, nb + 1, tshift, tsum);
+  cell_offsets_kernel<<<(unsigned)ntiles, kScanThreads, 0, st>>>(count, nb + 1, tshift, tsum, b.hist);
   launches++;
-  if (n > 0) {
+  if (n > 0 && slots) {
+    cell_place_kernel<<<ceil_div(n, 256), 256, 0, st>>>(n, b.keys[1], b.vals[1], b.rec, b.cell_start, bm, sl, b.tkeys,
+                                                        b.tmp, b.keys[0], b.vals[0], b.rec_sorted, b.hist);
+    launches++;
+  } else if (n > 0) {
     cell_scatter_kernel<<<ceil_div(n, 256), 256, 0, st>>>(n, b.keys[1], b.vals[1], b.rec, b.cell_start, bm,
                                                           b.keys[0], b.vals[0], b.tkeys, b.tmp, b.rec_sorted);
     cell_fixup_kernel<<<ceil_div(n, 256), 256, 0, st>>>(n, b.cell_start, bm, b.tkeys, b.tmp, b.keys[0], b.vals[0],
-                                                        b.rec, b.rec_sorted, ctl, b.hist);
+                                                        b.rec, b.rec_sorted);
     launches += 2;
   }
   return launches;

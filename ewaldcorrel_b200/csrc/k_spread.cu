@@ -476,7 +476,7 @@ int launch_spread(const Geom &g, const Spline &S, const int *cell_start, const u
   A.g = g;
   A.cs = cell_start;
   const long nb = sort_buckets(g, kSpreadZShift);
-  A.head = reinterpret_cast<const uint32_t *>(cell_start) + nb + 3;  // layout of cell_count_words
+  A.head = reinterpret_cast<const uint32_t *>(cell_start) + nb + 1;  // layout of cell_count_words
   A.tail = A.head + nb;
   A.keys = keys_sorted;
   A.rec = rec_sorted;

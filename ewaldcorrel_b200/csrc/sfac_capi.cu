@@ -232,6 +232,8 @@ void free_real(Handle *h) {
   }
   dfree(r.sb.tmp);
   dfree(r.sb.tkeys);
+  dfree(r.sb.next);
+  dfree(r.sb.slots);
   dfree(r.sb.rec);
   dfree(r.sb.rec_sorted);
   dfree(r.sb.hist);
@@ -253,11 +255,17 @@ bool ensure_real(Handle *h, int n, long ncell) {
   if (n <= r.cap && ncell == r.ncell && r.out) return true;
   const int cap = n > r.cap ? n + n / 2 + 64 : r.cap;
   free_real(h);
+  // slots for the sort while a cell's mean is small (12 points at water's
+  // density and a 1 nm cutoff): 2 mean + 6 of them, a multiple of 4
+  const double mean = (double)n / (double)ncell;
+  const bool slots = mean <= 28.0;
+  r.sb.nslot = slots ? ((int)(2.0 * mean) + 6 + 4) / 4 * 4 : 0;
   bool ok = true;
   for (int i = 0; i < 2 && ok; i++) ok = dalloc(h, &r.sb.keys[i], cap) && dalloc(h, &r.sb.vals[i], cap);
   ok = ok && dalloc(h, &r.sb.tmp, cap) && dalloc(h, &r.sb.tkeys, cap) && dalloc(h, &r.sb.rec, cap) &&
        dalloc(h, &r.sb.rec_sorted, cap) &&
-       dalloc(h, &r.sb.hist, cap) && dalloc(h, &r.sb.cell_start, cell_count_words(ncell)) &&
+       dalloc(h, &r.sb.hist, cap) && dalloc(h, &r.sb.cell_start, cell_count_words(ncell, slots)) &&
+       (!slots || (dalloc(h, &r.sb.slots, (size_t)r.sb.nslot * ncell) && dalloc(h, &r.sb.next, cap))) &&
        dalloc(h, &r.rec, cap) && dalloc(h, &r.x, 3 * (size_t)cap) && dalloc(h, &r.w, cap) &&
        dalloc(h, &r.dx, 3 * (size_t)cap) && dalloc(h, &r.part, real_partial_words(cap)) && dalloc(h, &r.out, 16) &&
        dalloc(h, &r.tab, kRealTab);
@@ -279,6 +287,7 @@ void free_atoms(Handle *h) {
   }
   dfree(h->sb.tmp);
   dfree(h->sb.tkeys);
+  dfree(h->sb.next);
   dfree(h->sb.rec);
   dfree(h->sb.rec_sorted);
   dfree(h->sb.hist);
@@ -291,7 +300,8 @@ bool ensure_atoms(Handle *h, int n) {
   const int cap = n + n / 2 + 64;
   bool ok = dalloc(h, &h->d_x, 3 * (size_t)cap) && dalloc(h, &h->d_w, cap);
   for (int i = 0; i < 2; i++) ok = ok && dalloc(h, &h->sb.keys[i], cap) && dalloc(h, &h->sb.vals[i], cap);
-  ok = ok && dalloc(h, &h->sb.tmp, cap) && dalloc(h, &h->sb.tkeys, cap) && dalloc(h, &h->sb.rec, cap) &&
+  ok = ok && dalloc(h, &h->sb.tmp, cap) && dalloc(h, &h->sb.tkeys, cap) && dalloc(h, &h->sb.next, cap) &&
+       dalloc(h, &h->sb.rec, cap) &&
        dalloc(h, &h->sb.rec_sorted, cap) &&
        dalloc(h, &h->sb.hist, cap);
   if (!ok) {
@@ -419,6 +429,7 @@ void *sfac_ctor(double L[6], int K[3], int order) {
   g.order = order;
   make_spline(order, h->spline, h->nodes);
   fft_prepare_kernels();
+  sort_prepare();
   spread_prepare();
   gather_prepare();
   if (const char *e = getenv("SFAC_NO_GRAPH")) h->use_graph = !(e[0] && e[0] != '0');
@@ -431,18 +442,23 @@ void *sfac_ctor(double L[6], int K[3], int order) {
             CK(h, cudaEventCreateWithFlags(&h->ev_in, cudaEventDisableTiming));
   h->stream = h->own_stream;
   for (int i = 0; i < 7 && ok; i++) ok = CK(h, cudaEventCreate(&h->ev_stage[i]));
-  ok = ok && dalloc(h, &h->d_real, h->nreal) && dalloc(h, &h->d_cplx, h->nmodes) &&
+  // the real grid also serves as the sort's slots (before the spread writes it)
+  const size_t slot_words = 2 * kSpreadSlots * (size_t)sort_buckets(g, kSpreadZShift);
+  ok = ok && dalloc(h, &h->d_real, slot_words > (size_t)h->nreal ? slot_words : (size_t)h->nreal) &&
+       dalloc(h, &h->d_cplx, h->nmodes) &&
        dalloc(h, &h->d_partials,
               (size_t)(fft_x_blocks_max(K[1], K[2]) > kConvBlocks ? fft_x_blocks_max(K[1], K[2]) : kConvBlocks) *
                   kRedWords) &&
        dalloc(h, &h->d_red, kRedWords) && dalloc(h, &h->d_ev, kRedWords) && dalloc(h, &h->d_cell, 1) &&
        dalloc(h, &h->d_ic, 1) &&
-       dalloc(h, &h->sb.cell_start, cell_count_words(sort_buckets(g, kSpreadZShift)));
+       dalloc(h, &h->sb.cell_start, cell_count_words(sort_buckets(g, kSpreadZShift), true));
   for (int d = 0; d < 3 && ok; d++) ok = dalloc(h, &h->d_iB[d], K[d]) && dalloc(h, &h->d_tw[d], K[d]);
   const size_t hf = (size_t)(2 * h->nmodes > h->nreal ? 2 * h->nmodes : h->nreal);
   ok = ok && CK(h, cudaMallocHost((void **)&h->h_S, sizeof(double) * 2 * h->nmodes)) &&
        CK(h, cudaMallocHost((void **)&h->h_f, sizeof(float) * hf)) &&
        CK(h, cudaMallocHost((void **)&h->h_red, sizeof(double) * kRedWords));
+  h->sb.slots = reinterpret_cast<uint2 *>(h->d_real);
+  h->sb.nslot = kSpreadSlots;
   if (ok) {
     g.cell = h->d_cell;
     ok = set_cell(h, L);
@@ -1194,10 +1210,10 @@ unsigned long sfac_footprint_bytes(const int K[3], int n) {
   const size_t K0 = K[0], K1 = K[1], K2 = K[2], ldim = K2 / 2 + 1, nn = (size_t)(n > 0 ? n : 1);
   const size_t cap = nn + nn / 2 + 64;
   const long nzb = ((long)K2 + (1L << kSpreadZShift) - 1) >> kSpreadZShift;
-  size_t b = 4 * K0 * K1 * K2 + 8 * K0 * K1 * ldim + 4 * cell_count_words((long)(K0 * K1) * nzb);  // grids, buckets
+  size_t b = 8 * kSpreadSlots * K0 * K1 * nzb + 8 * K0 * K1 * ldim + 4 * cell_count_words((long)(K0 * K1) * nzb, true);  // grids, buckets
   b += (K0 + K1 + K2) * 16 + sizeof(RowImg) * K0 * K1;                   // moduli, twiddles, rows
   b += 8 * (size_t)fft_x_blocks_max(K[1], K[2]) * kRedWords;               // partials
-  b += cap * (24 + 8 + 7 * 4 + 16 + 16);                                   // sort buffers, records
+  b += cap * (24 + 8 + 8 * 4 + 16 + 16);                                   // sort buffers, records
   b += 8 * cap * 8;                                                        // gather staging
   b += 8 * 2 * K0 * K1 * ldim + 4 * K0 * K1 * K2;                          // host mirrors (pinned)
   return b;
