@@ -622,192 +622,140 @@ __global__ void __launch_bounds__(512) fft_y2_kernel(int n, int n1, int n2, cons
   }
 }
 
-// Copies the contiguous block src[0 .. valid) (elements of T in rows of
-// `width`) into sh[r * pitch + c] for the first `total` elements, zero past
-// `valid`.  16-byte loads, four per thread issued before any of them is
-// stored, so that a small CTA keeps many loads in flight (a row-by-row loop
-// whose stores wait on each load leaves one in flight per thread); the row
-// and column of each element are advanced incrementally.  src must be
-// 16-byte aligned.
-template <typename T>
-__device__ __forceinline__ void stage_rows(const T *__restrict__ src, int valid, int total, int width, int pitch,
-                                           T *sh) {
-  constexpr int PER = 16 / sizeof(T);
-  const int nv = (total + PER - 1) / PER;
-  const int step = PER * blockDim.x;  // elements per pass of the CTA
-  const int sr = step / width, sc = step - sr * width;
-  int r = (PER * threadIdx.x) / width, c = PER * threadIdx.x - r * width;
-  for (int i = threadIdx.x; i < nv; i += 4 * blockDim.x) {
-    float4 v[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const int iu = i + u * blockDim.x, f = iu * PER;
-      if (iu < nv && f + PER <= valid) {
-        v[u] = __ldg(reinterpret_cast<const float4 *>(src) + iu);
-      } else {
-        T *e = reinterpret_cast<T *>(&v[u]);
-#pragma unroll
-        for (int k = 0; k < PER; k++) e[k] = (iu < nv && f + k < valid) ? src[f + k] : T{};
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const int iu = i + u * blockDim.x;
-      if (iu < nv) {
-        const T *e = reinterpret_cast<const T *>(&v[u]);
-        int rr = r, cc = c;
-#pragma unroll
-        for (int k = 0; k < PER; k++) {
-          if (iu * PER + k < total) sh[rr * pitch + cc] = e[k];
-          if (++cc == width) {
-            cc = 0;
-            rr++;
-          }
-        }
-      }
-      r += sr;
-      c += sc;
-      if (c >= width) {
-        c -= width;
-        r++;
-      }
-    }
+// z passes.  A group of G = 8 or 16 lanes (the power of two that holds both
+// factors) transforms one complex line, row[2b] + i row[2b+1], in registers:
+// lane t runs step-1 task j2 = t and step-2 task k1 = t.  The rows go straight
+// between global memory and the registers (consecutive lanes take consecutive
+// elements of a row, 32 to 64 bytes at a time), the two steps exchange through
+// the warp's own shared memory (element (k1, j2) at k1 (n2 + 1) + j2: no bank
+// conflicts in either direction) and no step waits for another warp.  Staging
+// the rows in shared memory, and the result again for the split into two
+// rows, took 2.9 times the shared-memory wavefronts and five CTA barriers.
+constexpr int kZWarps = 4;  // most warps per CTA
+
+// Twiddles in the order of the exchange: twx[k1 n2 + j2] = tw[j2 k1].
+__device__ __forceinline__ void load_twx(float2 *twx, const float2 *__restrict__ tw, int n, int n2) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const int k1 = i / n2, j2 = i - k1 * n2;
+    twx[i] = tw[j2 * k1];
   }
 }
 
-// z pass, real to half-complex: 2B consecutive real rows of length n per
-// CTA (row pair b forms the complex line row[2b] + i row[2b+1]); the rows
-// are read and the ldim = n/2 + 1 outputs written as contiguous blocks.
-// Shared: tw[n] | ex[B*n] | rows (2B x (n+1) floats), later Z (B x (n+1) complex).
-__global__ void __launch_bounds__(512) fft_zr2c2_kernel(int n, int n1, int n2, const float2 *__restrict__ twg,
-                                                        const float *__restrict__ rin, float2 *__restrict__ cout,
-                                                        long nrows, int lgB) {
+// Forward: real rows of length n -> ldim = n/2 + 1 outputs each.
+template <int G>
+__global__ void __launch_bounds__(32 * kZWarps) fft_z2_r2c_kernel(int n, int n1, int n2,
+                                                                  const float2 *__restrict__ twg,
+                                                                  const float *__restrict__ rin,
+                                                                  float2 *__restrict__ cout, int nrows) {
   extern __shared__ float2 sm[];
-  const int B = 1 << lgB, ldim = n / 2 + 1, RP = n + 1, ZP = n + 1;
-  float2 *tw = sm, *ex = sm + n, *Z = ex + B * n;
-  float *rows = reinterpret_cast<float *>(Z);
-  for (int i = threadIdx.x; i < n; i += blockDim.x) tw[i] = twg[i];
-  const long row0 = (long)blockIdx.x * 2 * B;
-  const int nr = (int)min((long)(2 * B), nrows - row0);
-  const float *src = rin + row0 * n;
-  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-    stage_rows<float>(src, nr * n, 2 * B * n, n, RP, rows);
-  } else {
-    for (int rr = threadIdx.x >> 5; rr < 2 * B; rr += nw)
-      for (int j = lane; j < n; j += 32) rows[rr * RP + j] = (rr < nr) ? src[(long)rr * n + j] : 0.f;
-  }
-  __syncthreads();
-  const int b = threadIdx.x & (B - 1), t = threadIdx.x >> lgB;
-  if (t < n2) {
-    const int j2 = t;
-    const float *ra = rows + (2 * b) * RP, *rb = ra + RP;
-    rdft::with_radix(n1, [&](auto RI) {
-      constexpr int R = decltype(RI)::value;
-      float2 u[R];
+  constexpr int LW = 32 / G;  // lines per warp
+  const int ldim = n / 2 + 1, exn = n1 * (n2 + 1);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = lane & (G - 1);
+  const int line = (blockIdx.x * (blockDim.x >> 5) + warp) * LW + lane / G;
+  float2 *twx = sm, *ex = sm + n + (warp * LW + lane / G) * exn;
+  const int ra = 2 * line, rb = ra + 1;
+  const bool la = ra < nrows && t < n2, lb = rb < nrows && t < n2;
+  const float *pa = rin + (long)ra * n + t, *pb = pa + n;
+  load_twx(twx, twg, n, n2);
+  rdft::with_radix(n1, [&](auto RI) {
+    constexpr int R = decltype(RI)::value;
+    float2 u[R];
 #pragma unroll
-      for (int j1 = 0; j1 < R; j1++) u[j1] = make_float2(ra[j2 + n2 * j1], rb[j2 + n2 * j1]);
+    for (int j1 = 0; j1 < R; j1++) {
+      u[j1].x = la && SPME_IN(t + n2 * j1, n, CK_FFT_LINE) ? __ldg(pa + n2 * j1) : 0.f;
+      u[j1].y = lb && SPME_IN(t + n2 * j1, n, CK_FFT_LINE) ? __ldg(pb + n2 * j1) : 0.f;
+    }
+    __syncthreads();
+    if (t < n2) {
       rdft::dft<R, -1>(u);
 #pragma unroll
-      for (int k1 = 0; k1 < R; k1++) ex[(k1 * n2 + j2) * B + b] = cmul(u[k1], tw[j2 * k1]);
-    });
-  }
-  __syncthreads();
-  if (t < n1) {
-    const int k1 = t;
-    rdft::with_radix(n2, [&](auto RI) {
-      constexpr int R = decltype(RI)::value;
-      float2 w[R];
-#pragma unroll
-      for (int j2 = 0; j2 < R; j2++) w[j2] = ex[(k1 * n2 + j2) * B + b];
-      rdft::dft<R, -1>(w);
-#pragma unroll
-      for (int k2 = 0; k2 < R; k2++)
-        if (SPME_IN(k1 + n1 * k2, n, CK_FFT_LINE)) Z[b * ZP + k1 + n1 * k2] = w[k2];
-    });
-  }
-  __syncthreads();
-  float2 *dst = cout + row0 * ldim;
-  for (int rr = threadIdx.x >> 5; rr < nr; rr += nw) {
-    const float2 *zb = Z + (rr >> 1) * ZP;
-    for (int k = lane; k < ldim; k += 32) {
-      const float2 u = zb[k], v = zb[k == 0 ? 0 : n - k];
-      dst[(long)rr * ldim + k] = (rr & 1) ? make_float2(0.5f * (u.y + v.y), -0.5f * (u.x - v.x))
-                                          : make_float2(0.5f * (u.x + v.x), 0.5f * (u.y - v.y));
+      for (int k1 = 0; k1 < R; k1++) ex[k1 * (n2 + 1) + t] = cmul(u[k1], twx[k1 * n2 + t]);
     }
-  }
+  });
+  __syncwarp();
+  const int t1 = min(t, n1 - 1);                                // lanes past n1 repeat the last task
+  const int mirror = lane - t + (t1 == 0 ? 0 : n1 - t1);        // lane that holds the bins n - k
+  rdft::with_radix(n2, [&](auto RI) {
+    constexpr int R = decltype(RI)::value;
+    float2 w[R];
+#pragma unroll
+    for (int j2 = 0; j2 < R; j2++) w[j2] = ex[t1 * (n2 + 1) + j2];
+    rdft::dft<R, -1>(w);
+    // bin k = k1 + n1 k2 of the two rows from Z[k] and Z[n - k]
+#pragma unroll
+    for (int k2 = 0; k2 <= R / 2; k2++) {
+      if (k2 >= R) break;  // R = 1
+      float2 v;
+      v.x = __shfl_sync(0xffffffffu, w[R - 1 - k2].x, mirror);
+      v.y = __shfl_sync(0xffffffffu, w[R - 1 - k2].y, mirror);
+      if (t1 == 0) v = w[(R - k2) % R];
+      const float2 u = w[k2];
+      const int k = t + n1 * k2;
+      if (t < n1 && k < ldim) {
+        if (ra < nrows) cout[(long)ra * ldim + k] = make_float2(0.5f * (u.x + v.x), 0.5f * (u.y - v.y));
+        if (rb < nrows) cout[(long)rb * ldim + k] = make_float2(0.5f * (u.y + v.y), -0.5f * (u.x - v.x));
+      }
+    }
+  });
 }
 
-// z pass, half-complex to real: the inverse of fft_zr2c2_kernel.  The
-// complex line of row pair b is X_2b + i X_2b+1 over the full length (the
-// Hermitian extension; self-conjugate bins keep their real parts only, as a
-// c2r transform ignores their imaginary parts).
-// Shared: tw[n] | ex[B*n] | H (2B x (ldim+1) complex), later rows (2B x (n+1) floats).
-__global__ void __launch_bounds__(512) fft_zc2r2_kernel(int n, int n1, int n2, const float2 *__restrict__ twg,
-                                                        const float2 *__restrict__ cin, float *__restrict__ rout,
-                                                        long nrows, int lgB) {
+// Inverse: the complex line of row pair b is X_2b + i X_2b+1 over the full
+// length (the Hermitian extension; self-conjugate bins keep their real parts
+// only, as a c2r transform ignores their imaginary parts).
+template <int G>
+__global__ void __launch_bounds__(32 * kZWarps) fft_z2_c2r_kernel(int n, int n1, int n2,
+                                                                  const float2 *__restrict__ twg,
+                                                                  const float2 *__restrict__ cin,
+                                                                  float *__restrict__ rout, int nrows) {
   extern __shared__ float2 sm[];
-  const int B = 1 << lgB, ldim = n / 2 + 1, HP = ldim + 1, RP = n + 1;
-  float2 *tw = sm, *ex = sm + n, *H = ex + B * n;
-  float *rows = reinterpret_cast<float *>(H);
-  for (int i = threadIdx.x; i < n; i += blockDim.x) tw[i] = twg[i];
-  const long row0 = (long)blockIdx.x * 2 * B;
-  const int nr = (int)min((long)(2 * B), nrows - row0);
-  const float2 *src = cin + row0 * ldim;
-  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-    stage_rows<float2>(src, nr * ldim, 2 * B * ldim, ldim, HP, H);
-  } else {
-    for (int rr = threadIdx.x >> 5; rr < 2 * B; rr += nw)
-      for (int k = lane; k < ldim; k += 32)
-        H[rr * HP + k] = (rr < nr) ? src[(long)rr * ldim + k] : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
-  const int b = threadIdx.x & (B - 1), t = threadIdx.x >> lgB;
-  if (t < n2) {
-    const int j2 = t;
-    const float2 *ha = H + (2 * b) * HP, *hb = ha + HP;
-    rdft::with_radix(n1, [&](auto RI) {
-      constexpr int R = decltype(RI)::value;
-      float2 u[R];
+  constexpr int LW = 32 / G;
+  const int ldim = n / 2 + 1, exn = n1 * (n2 + 1);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = lane & (G - 1);
+  const int line = (blockIdx.x * (blockDim.x >> 5) + warp) * LW + lane / G;
+  float2 *twx = sm, *ex = sm + n + (warp * LW + lane / G) * exn;
+  const int ra = 2 * line, rb = ra + 1;
+  const bool la = ra < nrows && t < n2, lb = rb < nrows && t < n2;
+  const float2 *pa = cin + (long)ra * ldim, *pb = pa + ldim;
+  load_twx(twx, twg, n, n2);
+  rdft::with_radix(n1, [&](auto RI) {
+    constexpr int R = decltype(RI)::value;
+    float2 u[R];
 #pragma unroll
-      for (int j1 = 0; j1 < R; j1++) {
-        const int k = j2 + n2 * j1;
-        const bool lo = k < ldim;
-        const int kk = lo ? k : n - k;
-        float2 a = ha[kk], c = hb[kk];
-        if (kk == 0 || 2 * kk == n) {
-          a.y = 0.f;
-          c.y = 0.f;
-        }
-        u[j1] = lo ? make_float2(a.x - c.y, a.y + c.x) : make_float2(a.x + c.y, c.x - a.y);
+    for (int j1 = 0; j1 < R; j1++) {
+      const int k = t + n2 * j1;
+      const bool lo = k < ldim;
+      const int kk = lo ? k : n - k;
+      float2 a = make_float2(0.f, 0.f), c = make_float2(0.f, 0.f);
+      if (la && SPME_IN(kk, ldim, CK_FFT_LINE)) a = __ldg(pa + kk);
+      if (lb && SPME_IN(kk, ldim, CK_FFT_LINE)) c = __ldg(pb + kk);
+      if (kk == 0 || 2 * kk == n) {
+        a.y = 0.f;
+        c.y = 0.f;
       }
+      u[j1] = lo ? make_float2(a.x - c.y, a.y + c.x) : make_float2(a.x + c.y, c.x - a.y);
+    }
+    __syncthreads();
+    if (t < n2) {
       rdft::dft<R, +1>(u);
 #pragma unroll
-      for (int k1 = 0; k1 < R; k1++) ex[(k1 * n2 + j2) * B + b] = cmul(u[k1], twid<+1>(tw, j2 * k1));
-    });
-  }
-  __syncthreads();
-  if (t < n1) {
-    const int k1 = t;
-    float *ra = rows + (2 * b) * RP, *rb = ra + RP;
-    rdft::with_radix(n2, [&](auto RI) {
-      constexpr int R = decltype(RI)::value;
-      float2 w[R];
+      for (int k1 = 0; k1 < R; k1++) ex[k1 * (n2 + 1) + t] = cmul(u[k1], twid<+1>(twx, k1 * n2 + t));
+    }
+  });
+  __syncwarp();
+  if (t >= n1) return;
+  rdft::with_radix(n2, [&](auto RI) {
+    constexpr int R = decltype(RI)::value;
+    float2 w[R];
 #pragma unroll
-      for (int j2 = 0; j2 < R; j2++) w[j2] = ex[(k1 * n2 + j2) * B + b];
-      rdft::dft<R, +1>(w);
+    for (int j2 = 0; j2 < R; j2++) w[j2] = ex[t * (n2 + 1) + j2];
+    rdft::dft<R, +1>(w);
+    float *qa = rout + (long)ra * n + t, *qb = qa + n;
 #pragma unroll
-      for (int k2 = 0; k2 < R; k2++) {
-        ra[k1 + n1 * k2] = w[k2].x;
-        rb[k1 + n1 * k2] = w[k2].y;
-      }
-    });
-  }
-  __syncthreads();
-  float *dst = rout + row0 * n;
-  for (int rr = threadIdx.x >> 5; rr < nr; rr += nw)
-    for (int j = lane; j < n; j += 32) dst[(long)rr * n + j] = rows[rr * RP + j];
+    for (int k2 = 0; k2 < R; k2++) {
+      if (ra < nrows && SPME_IN(t + n1 * k2, n, CK_FFT_LINE)) qa[n1 * k2] = w[k2].x;
+      if (rb < nrows && SPME_IN(t + n1 * k2, n, CK_FFT_LINE)) qb[n1 * k2] = w[k2].y;
+    }
+  });
 }
 
 // FP32 twiddles exp(-2 pi i k / n), evaluated in FP64.
@@ -873,8 +821,6 @@ void fft_prepare_kernels() {
   for (const void *f : x2) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute((const void *)fft_y2_kernel<-1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute((const void *)fft_y2_kernel<+1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute((const void *)fft_zr2c2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute((const void *)fft_zc2r2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
 }
 
 // Shared memory of the plane kernels: twiddles + two buffers of `sz`.
@@ -912,6 +858,28 @@ static bool lines2_shape(int n, long nlines, int min_threads, int &n1, int &n2, 
   return true;
 }
 
+// Two-level z pass over nrows rows of length n: groups of 8 or 16 lanes, and
+// fewer warps per CTA while the SMs would not all get one.
+template <bool FWD>
+static void launch_z2(int n, const float2 *tw, float *real, float2 *cplx, int nrows, cudaStream_t st) {
+  int n1, n2;
+  rdft::split_line(n, n1, n2);
+  const bool small = n1 <= 8;  // n2 <= n1
+  const int lw = small ? 4 : 2;
+  const long warps = ((long)(nrows + 1) / 2 + lw - 1) / lw;
+  int wpc = kZWarps;
+  while (wpc > 1 && warps < 148L * wpc) wpc >>= 1;
+  const size_t smem = (size_t)(n + wpc * lw * n1 * (n2 + 1)) * sizeof(float2);
+  const unsigned blocks = (unsigned)((warps + wpc - 1) / wpc);
+  if (FWD) {
+    if (small) fft_z2_r2c_kernel<8><<<blocks, 32 * wpc, smem, st>>>(n, n1, n2, tw, real, cplx, nrows);
+    else fft_z2_r2c_kernel<16><<<blocks, 32 * wpc, smem, st>>>(n, n1, n2, tw, real, cplx, nrows);
+  } else {
+    if (small) fft_z2_c2r_kernel<8><<<blocks, 32 * wpc, smem, st>>>(n, n1, n2, tw, cplx, real, nrows);
+    else fft_z2_c2r_kernel<16><<<blocks, 32 * wpc, smem, st>>>(n, n1, n2, tw, cplx, real, nrows);
+  }
+}
+
 // Which z/y implementation a plan uses: the fused plane kernels (an x-plane
 // in shared memory), the two-level per-axis passes, or the Stockham
 // per-axis passes (any length).
@@ -943,14 +911,10 @@ int fwd_zy(const FftPlan3 &F, const float *real, float2 *cplx, cudaStream_t st) 
   const long nl = (long)K0 * ldim;
   if (zy == ZY_TWO_LEVEL) {
     int n1, n2, lgB, thr;
-    lines2_shape(K2, (nrows + 1) / 2, 0, n1, n2, lgB, thr);
-    int B = 1 << lgB;
-    size_t smem = (size_t)(K2 + (size_t)B * K2 + (size_t)B * (K2 + 4)) * sizeof(float2);
-    fft_zr2c2_kernel<<<(unsigned)((nrows + 2 * B - 1) / (2 * B)), thr, smem, st>>>(K2, n1, n2, F.len[2].tw, real,
-                                                                                  cplx, nrows, lgB);
+    launch_z2<true>(K2, F.len[2].tw, const_cast<float *>(real), cplx, (int)nrows, st);
     lines2_shape(K1, nl, 0, n1, n2, lgB, thr);
-    B = 1 << lgB;
-    smem = (size_t)(K1 + (size_t)B * K1) * sizeof(float2);
+    const int B = 1 << lgB;
+    const size_t smem = (size_t)(K1 + (size_t)B * K1) * sizeof(float2);
     fft_y2_kernel<-1><<<(unsigned)((nl + B - 1) / B), thr, smem, st>>>(K1, n1, n2, F.len[1].tw, cplx, nl,
                                                                        FastDiv(ldim), (long)K1 * ldim, ldim, lgB,
                                                                        nullptr, 0, nullptr, nullptr, nullptr);
@@ -988,16 +952,12 @@ int inv_yz(const FftPlan3 &F, float2 *cplx, float *real, const double *partials,
   if (zy == ZY_TWO_LEVEL) {
     int n1, n2, lgB, thr;
     lines2_shape(K1, nl, partials ? 256 : 0, n1, n2, lgB, thr);
-    int B = 1 << lgB;
-    size_t smem = (size_t)(K1 + (size_t)B * K1) * sizeof(float2);
+    const int B = 1 << lgB;
+    const size_t smem = (size_t)(K1 + (size_t)B * K1) * sizeof(float2);
     fft_y2_kernel<+1><<<(unsigned)((nl + B - 1) / B), thr, smem, st>>>(K1, n1, n2, F.len[1].tw, cplx, nl,
                                                                        FastDiv(ldim), (long)K1 * ldim, ldim, lgB,
                                                                        partials, nblocks, cell, raw, ev);
-    lines2_shape(K2, (nrows + 1) / 2, 0, n1, n2, lgB, thr);
-    B = 1 << lgB;
-    smem = (size_t)(K2 + (size_t)B * K2 + (size_t)B * (K2 + 4)) * sizeof(float2);
-    fft_zc2r2_kernel<<<(unsigned)((nrows + 2 * B - 1) / (2 * B)), thr, smem, st>>>(K2, n1, n2, F.len[2].tw, cplx,
-                                                                                  real, nrows, lgB);
+    launch_z2<false>(K2, F.len[2].tw, real, cplx, (int)nrows, st);
     return 2;
   }
   int k = 0;
