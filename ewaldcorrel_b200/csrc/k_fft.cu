@@ -362,6 +362,14 @@ __global__ void __launch_bounds__(256) fft_x_kernel(FftLen L, Geom g, Influence 
   }
 }
 
+// Twiddles in the order of the exchange: twx[k1 n2 + j2] = tw[j2 k1].
+__device__ __forceinline__ void load_twx(float2 *twx, const float2 *__restrict__ tw, int n, int n2) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const int k1 = i / n2, j2 = i - k1 * n2;
+    twx[i] = tw[j2 * k1];
+  }
+}
+
 // --- x pass, two-level register transform ---------------------------------
 // Same modes and results as fft_x_kernel, for K0 = n1 * n2 with n1, n2 <= 16.
 // B lines per CTA (a power of two, lines b fastest in the thread index so
@@ -376,18 +384,23 @@ __global__ void __launch_bounds__(512) fft_x2_kernel(int n, int n1, int n2, cons
                                                      Influence inf, const double *__restrict__ iB0,
                                                      const double *__restrict__ iB1, const double *__restrict__ iB2,
                                                      float2 *__restrict__ data, int lgB,
-                                                     double *__restrict__ partials) {
+                                                     double *__restrict__ partials, FastDiv ldd) {
   extern __shared__ float2 sm[];
   __shared__ double red[16][7];
   const int B = 1 << lgB;
-  float2 *tw = sm, *ex = sm + n;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) tw[i] = twg[i];
+  float2 *twx = sm, *ex = sm + n;
+  load_twx(twx, twg, n, n2);
   const int ldim = g.ldim, K1 = g.K1;
-  const long nlines = (long)K1 * ldim;
+  // 32-bit indices: the grid has fewer than 2^31 points, and the 64-bit
+  // divisions and products of an earlier version were a quarter of the pass's
+  // instructions (65 M -> 53 M and 130 -> 115 us at 256^3 without them)
+  const int nlines = K1 * ldim;
   const int b = threadIdx.x & (B - 1), t = threadIdx.x >> lgB;
-  const long line = (long)blockIdx.x * B + b;
+  const int line = blockIdx.x * B + b;
   const bool live = line < nlines;
-  const int ky = live ? (int)(line / ldim) : 0, kz = live ? (int)(line - (long)ky * ldim) : 0;
+  uint32_t uy = 0, uz = 0;
+  if (live) ldd.divmod((uint32_t)line, uy, uz);
+  const int ky = (int)uy, kz = (int)uz;
   constexpr bool FWD = (MODE == XM_FWD_DECONV || MODE == XM_FWD_CONV_INV);
   // compact influence table: the CTA's n x B entries are copied to shared
   // memory (abuf[kx * B + b]) with cp.async now and used after the forward
@@ -395,17 +408,14 @@ __global__ void __launch_bounds__(512) fft_x2_kernel(int n, int n1, int n2, cons
   double *abuf = reinterpret_cast<double *>(ex + (size_t)B * n);
   constexpr bool PREFETCH = (IM == 4 && MODE != XM_FWD_DECONV);
   if (PREFETCH) {
-    for (int e = threadIdx.x; e < B * n; e += blockDim.x) {
-      const int bb = e & (B - 1), kx = e >> lgB;
-      const long ln = (long)blockIdx.x * B + bb;
-      if (ln < nlines) {
-        const int y = (int)(ln / ldim), z = (int)(ln - (long)y * ldim);
-        const unsigned dst = (unsigned)__cvta_generic_to_shared(abuf + e);
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst),
-                     "l"(inf.A + ((long)kx * K1 + y) * ldim + z)
+    // a thread copies entries of its own line: no division per entry
+    const int step = blockDim.x >> lgB;
+    if (live)
+      for (int kx = t; kx < n; kx += step) {
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(abuf + kx * B + b);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(inf.A + (size_t)(kx * nlines + line))
                      : "memory");
       }
-    }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   __syncthreads();
@@ -416,11 +426,11 @@ __global__ void __launch_bounds__(512) fft_x2_kernel(int n, int n1, int n2, cons
       float2 u[R];
 #pragma unroll
       for (int j1 = 0; j1 < R; j1++)
-        u[j1] = (live && SPME_IN(j2 + n2 * j1, n, CK_FFT_LINE)) ? data[line + (long)(j2 + n2 * j1) * nlines]
+        u[j1] = (live && SPME_IN(j2 + n2 * j1, n, CK_FFT_LINE)) ? data[line + (j2 + n2 * j1) * nlines]
                                                                 : make_float2(0.f, 0.f);
       rdft::dft<R, -1>(u);
 #pragma unroll
-      for (int k1 = 0; k1 < R; k1++) ex[(k1 * n2 + j2) * B + b] = cmul(u[k1], tw[j2 * k1]);
+      for (int k1 = 0; k1 < R; k1++) ex[(k1 * n2 + j2) * B + b] = cmul(u[k1], twx[k1 * n2 + j2]);
     });
   }
   if (PREFETCH) asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -440,7 +450,7 @@ __global__ void __launch_bounds__(512) fft_x2_kernel(int n, int n1, int n2, cons
       } else {
 #pragma unroll
         for (int k2 = 0; k2 < R; k2++)
-          w[k2] = (live && SPME_IN(k1 + n1 * k2, n, CK_FFT_LINE)) ? data[line + (long)(k1 + n1 * k2) * nlines]
+          w[k2] = (live && SPME_IN(k1 + n1 * k2, n, CK_FFT_LINE)) ? data[line + (k1 + n1 * k2) * nlines]
                                                                   : make_float2(0.f, 0.f);
       }
       if (MODE == XM_FWD_DECONV) {
@@ -449,7 +459,7 @@ __global__ void __launch_bounds__(512) fft_x2_kernel(int n, int n1, int n2, cons
 #pragma unroll
           for (int k2 = 0; k2 < R; k2++) {
             const int kx = k1 + n1 * k2;
-            if (SPME_IN(kx, n, CK_FFT_LINE)) data[line + (long)kx * nlines] = cscale(w[k2], (float)(iB0[kx] * s12));
+            if (SPME_IN(kx, n, CK_FFT_LINE)) data[line + kx * nlines] = cscale(w[k2], (float)(iB0[kx] * s12));
           }
         }
       } else if (IM == 1) {
@@ -462,9 +472,7 @@ __global__ void __launch_bounds__(512) fft_x2_kernel(int n, int n1, int n2, cons
 #pragma unroll
           for (int k2 = 0; k2 < R; k2++) {
             const int kx = k1 + n1 * k2;
-            const long i = SPME_IN(((long)kx * K1 + ky) * ldim + kz, (long)n * K1 * ldim, CK_FFT_CONV)
-                               ? ((long)kx * K1 + ky) * ldim + kz
-                               : 0;
+            const int i = SPME_IN(kx * nlines + line, n * nlines, CK_FFT_CONV) ? kx * nlines + line : 0;
             const float2 q = w[k2];
             const double ib = iB0[kx] * s12;
             double sq = (double)q.x * q.x + (double)q.y * q.y;
@@ -472,7 +480,7 @@ __global__ void __launch_bounds__(512) fft_x2_kernel(int n, int n1, int n2, cons
             const double A = inf.A[i];
             acc[0] += sq * A;
 #pragma unroll
-            for (int c = 0; c < 6; c++) acc[1 + c] += sq * inf.dA[6 * i + c];
+            for (int c = 0; c < 6; c++) acc[1 + c] += sq * inf.dA[6 * (size_t)i + c];
             if (MODE != XM_EN) {
               double f = A * ib * (MODE == XM_FWD_CONV_INV ? ib : 1.0);
               if (plane) f *= 2.0;
@@ -484,7 +492,7 @@ __global__ void __launch_bounds__(512) fft_x2_kernel(int n, int n1, int n2, cons
           rdft::dft<R, +1>(w);
 #pragma unroll
           for (int j2 = 0; j2 < R; j2++) {
-            float2 c = tw[j2 * k1];
+            float2 c = twx[k1 * n2 + j2];
             c.y = -c.y;
             ex[(k1 * n2 + j2) * B + b] = cmul(w[j2], c);
           }
@@ -503,9 +511,7 @@ __global__ void __launch_bounds__(512) fft_x2_kernel(int n, int n1, int n2, cons
 #pragma unroll 1
           for (int k2 = 0; k2 < R; k2++) {
             const int kx = k1 + n1 * k2;
-            const long i = SPME_IN(((long)kx * K1 + ky) * ldim + kz, (long)n * K1 * ldim, CK_FFT_CONV)
-                               ? ((long)kx * K1 + ky) * ldim + kz
-                               : 0;
+            const int i = SPME_IN(kx * nlines + line, n * nlines, CK_FFT_CONV) ? kx * nlines + line : 0;
             const float2 q = slot[k2 * B];
             const double ib = iB0[kx] * s12;
             double sq = (double)q.x * q.x + (double)q.y * q.y;
@@ -526,7 +532,7 @@ __global__ void __launch_bounds__(512) fft_x2_kernel(int n, int n1, int n2, cons
           rdft::dft<R, +1>(w);
 #pragma unroll
           for (int j2 = 0; j2 < R; j2++) {
-            float2 c = tw[j2 * k1];
+            float2 c = twx[k1 * n2 + j2];
             c.y = -c.y;
             ex[(k1 * n2 + j2) * B + b] = cmul(w[j2], c);
           }
@@ -560,7 +566,7 @@ __global__ void __launch_bounds__(512) fft_x2_kernel(int n, int n1, int n2, cons
       rdft::dft<R, +1>(u);
 #pragma unroll
       for (int j1 = 0; j1 < R; j1++)
-        if (SPME_IN(j2 + n2 * j1, n, CK_FFT_LINE)) data[line + (long)(j2 + n2 * j1) * nlines] = u[j1];
+        if (SPME_IN(j2 + n2 * j1, n, CK_FFT_LINE)) data[line + (j2 + n2 * j1) * nlines] = u[j1];
     });
   }
 }
@@ -632,14 +638,6 @@ __global__ void __launch_bounds__(512) fft_y2_kernel(int n, int n1, int n2, cons
 // the rows in shared memory, and the result again for the split into two
 // rows, took 2.9 times the shared-memory wavefronts and five CTA barriers.
 constexpr int kZWarps = 4;  // most warps per CTA
-
-// Twiddles in the order of the exchange: twx[k1 n2 + j2] = tw[j2 k1].
-__device__ __forceinline__ void load_twx(float2 *twx, const float2 *__restrict__ tw, int n, int n2) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int k1 = i / n2, j2 = i - k1 * n2;
-    twx[i] = tw[j2 * k1];
-  }
-}
 
 // Forward: real rows of length n -> ldim = n/2 + 1 outputs each.
 template <int G>
@@ -1030,7 +1028,7 @@ static int x_pass(const FftPlan3 &F, const Geom &g, const Influence &inf, const 
       constexpr int IM = decltype(IMC)::value;
       const size_t sm = smem + (IM == 4 && MODE != XM_FWD_DECONV ? (size_t)B * n * sizeof(double) : 0);
       fft_x2_kernel<MODE, IM><<<nblocks, threads, sm, st>>>(n, n1, n2, F.len[0].tw, g, inf, iB0, iB1, iB2, cplx,
-                                                            lgB, partials);
+                                                            lgB, partials, FastDiv((uint32_t)g.ldim));
     };
     if (MODE == XM_FWD_DECONV || inf.mode == 1) go(std::integral_constant<int, 1>{});
     else if (inf.mode == 4) go(std::integral_constant<int, 4>{});
