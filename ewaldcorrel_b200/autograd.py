@@ -11,7 +11,11 @@ only scales them by the incoming gradient.
 ``SpmeBatch`` evaluates many independent systems (different sizes, boxes and
 grids) in one call: every system keeps a plan with fixed device buffers, so
 its solve replays as a CUDA graph, and the solves run concurrently on the
-plans' own streams.
+plans' own streams.  The plans' buffers are slices of the batch's and one
+native call launches all solves (sfac_solve_device_many), so that the host
+cost per system is a graph launch and three event calls, not ten torch
+operations: 16 systems of 64 to 2048 charges, forward and backward, took
+1400 us of host time before.
 """
 from __future__ import annotations
 
@@ -29,6 +33,8 @@ def _lib():
     if not getattr(lib, "_autograd_declared", False):
         lib.sfac_solve_device_cell.argtypes = [c_void_p, c_int] + [c_void_p] * 6
         lib.sfac_solve_device_cell.restype = c_int
+        lib.sfac_solve_device_many.argtypes = [c_int] + [c_void_p] * 9
+        lib.sfac_solve_device_many.restype = c_int
         lib.sfac_get_stream.argtypes = [c_void_p]
         lib.sfac_get_stream.restype = c_void_p
         lib._autograd_declared = True
@@ -39,10 +45,11 @@ class SpmePlan:
     """One system shape (atom count, grid, order) with fixed device buffers.
 
     The box may change between calls (the influence function is re-set on
-    the device); inputs are copied into the plan's buffers so that the
-    solve's CUDA graph keeps valid pointers."""
+    the device); inputs are copied into the plan's buffers (its own, or a
+    batch's slices of common ones) so that the solve's CUDA graph keeps valid
+    pointers."""
 
-    def __init__(self, n, K, order=4, beta=3.47, max_m=None, L=None, device=None):
+    def __init__(self, n, K, order=4, beta=3.47, max_m=None, L=None, device=None, buffers=None):
         self.device = torch.device("cuda", torch.cuda.current_device() if device is None else device)
         self.n, self.K, self.order = int(n), tuple(int(k) for k in K), int(order)
         self.beta = float(beta)
@@ -54,13 +61,11 @@ class SpmePlan:
             self.L = L.copy()
             self.lib = _lib()
             self.stream = torch.cuda.ExternalStream(self.lib.sfac_get_stream(self.sf._data), device=self.device)
-            dev = self.device
-            self.x = torch.zeros((max(self.n, 1), 3), dtype=torch.float64, device=dev)
-            self.q = torch.zeros(max(self.n, 1), dtype=torch.float64, device=dev)
-            self.dx = torch.zeros((max(self.n, 1), 3), dtype=torch.float64, device=dev)
-            self.phi = torch.zeros(max(self.n, 1), dtype=torch.float64, device=dev)
-            self.ev = torch.zeros(7, dtype=torch.float64, device=dev)
-            self.dEdL = torch.zeros(6, dtype=torch.float64, device=dev)
+            if buffers is None:
+                m = max(self.n, 1)
+                buffers = [torch.zeros(shape, dtype=torch.float64, device=self.device)
+                           for shape in ((m, 3), (m,), (m, 3), (m,), (7,), (6,))]
+            self.x, self.q, self.dx, self.phi, self.ev, self.dEdL = buffers
         self.done = torch.cuda.Event()
 
     def set_box(self, L):
@@ -97,26 +102,11 @@ class _SpmeBatchFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, q, L, batch):
-        offs = batch.offsets
         cur = torch.cuda.current_stream(batch.device)
-        xd, qd = x.detach().to(batch.device, torch.float64), q.detach().to(batch.device, torch.float64)
-        ready = torch.cuda.Event()
-        ready.record(cur)
-        boxes = _box_numpy(L).reshape(-1, 6)
-        for i, p in enumerate(batch.plans):
-            p.set_box(boxes[i])
-            p.launch(xd[offs[i]:offs[i + 1]], qd[offs[i]:offs[i + 1]], ready)
-        B = len(batch.plans)
-        E = torch.empty(B, dtype=torch.float64, device=batch.device)
-        dx = torch.empty_like(xd)
-        phi = torch.empty_like(qd)
-        dL = torch.empty((B, 6), dtype=torch.float64, device=batch.device)
-        for i, p in enumerate(batch.plans):
-            cur.wait_event(p.done)
-            E[i : i + 1].copy_(p.ev[:1])
-            dx[offs[i]:offs[i + 1]].copy_(p.dx[: p.n])
-            phi[offs[i]:offs[i + 1]].copy_(p.phi[: p.n])
-            dL[i].copy_(p.dEdL)
+        with torch.cuda.device(batch.device), torch.cuda.stream(cur):
+            xd, qd = x.detach().to(batch.device, torch.float64), q.detach().to(batch.device, torch.float64)
+            batch.set_boxes(_box_numpy(L).reshape(-1, 6))
+            E, dx, phi, dL = batch.solve(xd, qd, cur)
         ctx.save_for_backward(dx, phi, dL)
         ctx.sysid = batch.sysid
         ctx.L_meta = (L.shape, L.device, L.dtype)
@@ -145,17 +135,54 @@ class SpmeBatch:
 
     def __init__(self, systems, beta=3.47, max_m=None, device=None):
         self.device = torch.device("cuda", torch.cuda.current_device() if device is None else device)
-        self.plans = []
-        counts = []
-        for s in systems:
-            n, K, order = s[0], s[1], s[2]
-            b = s[3] if len(s) > 3 else beta
-            mm = s[4] if len(s) > 4 else max_m
-            self.plans.append(SpmePlan(n, K, order, b, mm, device=self.device.index))
-            counts.append(int(n))
+        counts = [int(s[0]) for s in systems]
         self.offsets = [int(v) for v in np.concatenate([[0], np.cumsum(counts)])]
-        self.sysid = torch.repeat_interleave(torch.arange(len(counts), device=self.device),
-                                             torch.tensor(counts, device=self.device))
+        N, B = self.offsets[-1], len(counts)
+        with torch.cuda.device(self.device):
+            # the plans' buffers, back to back in the callers' layout: one copy in
+            # and one out serve all systems
+            new = lambda *shape: torch.zeros(shape, dtype=torch.float64, device=self.device)  # noqa: E731
+            self.x, self.q, self.dx, self.phi = new(N, 3), new(N), new(N, 3), new(N)
+            self.ev, self.dEdL = new(B, 7), new(B, 6)
+            self.plans = []
+            for i, s in enumerate(systems):
+                n, K, order = s[0], s[1], s[2]
+                b = s[3] if len(s) > 3 else beta
+                mm = s[4] if len(s) > 4 else max_m
+                o = slice(self.offsets[i], self.offsets[i + 1])
+                self.plans.append(SpmePlan(n, K, order, b, mm, device=self.device.index,
+                                           buffers=(self.x[o], self.q[o], self.dx[o], self.phi[o], self.ev[i],
+                                                    self.dEdL[i])))
+            self.sysid = torch.repeat_interleave(torch.arange(B, device=self.device),
+                                                 torch.tensor(counts, device=self.device))
+            self.boxes = np.stack([p.L for p in self.plans]) if B else np.zeros((0, 6))
+            self._n = np.asarray(counts, dtype=np.int32)
+            self._handles = (c_void_p * max(B, 1))(*[p.sf._data for p in self.plans])
+            self._lib = _lib()
+            self._free = torch.cuda.Event()  # the buffers' last use, on whatever stream it was
+            self._free.record(torch.cuda.current_stream(self.device))
+
+    def set_boxes(self, boxes):
+        """The boxes (B, 6) of the next solve; unchanged ones cost nothing."""
+        for i in np.nonzero((boxes != self.boxes).any(axis=1))[0]:
+            self.plans[i].set_box(boxes[i])
+            self.boxes[i] = boxes[i]
+
+    def solve(self, x, q, stream):
+        """Enqueues all systems' solves after `stream`'s work, on the plans' own
+        streams, and makes `stream` wait for them: (E, dE/dx, phi, dE/dL), new tensors."""
+        stream.wait_event(self._free)
+        self.x.copy_(x)
+        self.q.copy_(q)
+        rc = self._lib.sfac_solve_device_many(len(self.plans), self._handles, self._n.ctypes.data, self.x.data_ptr(),
+                                              self.q.data_ptr(), self.dx.data_ptr(), self.phi.data_ptr(),
+                                              self.ev.data_ptr(), self.dEdL.data_ptr(), c_void_p(stream.cuda_stream))
+        if rc != 0:
+            bad = self.plans[rc - 1].sf.last_error() if rc <= len(self.plans) else "event"
+            raise RuntimeError(f"sfac_solve_device_many failed ({rc}): {bad}")
+        out = self.ev[:, 0].clone(), self.dx.clone(), self.phi.clone(), self.dEdL.clone()
+        self._free.record(stream)
+        return out
 
     def __call__(self, x, q, L):
         return _SpmeBatchFn.apply(x, q, L, self)

@@ -76,6 +76,7 @@ struct Handle {
   cudaStream_t stream = nullptr;      // stream all work is enqueued on
   cudaStream_t own_stream = nullptr;  // the handle's own stream
   cudaEvent_t ev_in = nullptr;
+  cudaEvent_t ev_done = nullptr;      // end of a solve of sfac_solve_device_many (created on first use)
   cudaEvent_t ev_stage[7] = {};
   // device buffers
   float *d_real = nullptr;
@@ -367,6 +368,7 @@ void destroy(Handle *h) {
   if (h->h_f) cudaFreeHost(h->h_f);
   if (h->h_red) cudaFreeHost(h->h_red);
   if (h->ev_in) cudaEventDestroy(h->ev_in);
+  if (h->ev_done) cudaEventDestroy(h->ev_done);
   for (auto &e : h->ev_stage)
     if (e) cudaEventDestroy(e);
   if (h->graph) cudaGraphExecDestroy(h->graph);
@@ -1159,6 +1161,34 @@ int sfac_solve_device_cell(void *p, int n, const double *x, const double *w, dou
   Handle *h = H(p);
   if (!h || !dEdL) return 1;
   return solve_device(h, n, x, w, dx, phi, ev, dEdL, false);
+}
+
+int sfac_solve_device_many(int count, void *const *handles, const int *n, const double *x, const double *w, double *dx,
+                           double *phi, double *ev, double *dEdL, void *stream) {
+  if (count <= 0) return 0;
+  cudaStream_t cur = (cudaStream_t)stream;
+  Handle *first = H(handles[0]);
+  if (!first) return 1;
+  if (!CK(first, cudaEventRecord(first->ev_in, cur))) return 1;
+  int rc = 0, done = 0;
+  long a = 0;
+  for (int i = 0; i < count && rc == 0; i++) {
+    Handle *h = H(handles[i]);
+    if (!h || (!h->ev_done && !CK(h, cudaEventCreateWithFlags(&h->ev_done, cudaEventDisableTiming))) ||
+        !CK(h, cudaStreamWaitEvent(h->stream, first->ev_in, 0)) ||
+        solve_device(h, n[i], x + 3 * a, w + a, dx + 3 * a, phi + a, ev + 7 * i, dEdL + 6 * i, false) != 0 ||
+        !CK(h, cudaEventRecord(h->ev_done, h->stream))) {
+      rc = i + 1;
+      break;
+    }
+    done = i + 1;
+    a += n[i];
+  }
+  for (int i = 0; i < done; i++) {
+    Handle *h = H(handles[i]);
+    if (!CK(h, cudaStreamWaitEvent(cur, h->ev_done, 0)) && rc == 0) rc = i + 1;
+  }
+  return rc;
 }
 
 int sfac_solve_device_timed(void *p, int n, const double *x, const double *w, double *dx, double *phi,

@@ -180,6 +180,16 @@ int sfac_solve_device(void *sfac, int n, const double *x, const double *w, doubl
 int sfac_solve_device_cell(void *sfac, int n, const double *x, const double *w, double *dx, double *phi,
                            double *ev, double *dEdL);
 
+/* sfac_solve_device_cell of `count` handles of one device in one call, on
+ * each handle's own stream: x, w, dx and phi hold the systems back to back
+ * (n[i] atoms of system i), ev 7 and dEdL 6 doubles per system.  The solves
+ * start after the work already on `stream` (a cudaStream_t) and later work on
+ * it waits for them.  Returns 0, or 1 + the index of the system that failed
+ * (the later ones are not enqueued).  Not for two threads at once with a
+ * common handle. */
+int sfac_solve_device_many(int count, void *const *handles, const int *n, const double *x, const double *w, double *dx,
+                           double *phi, double *ev, double *dEdL, void *stream);
+
 /* The same solve with CUDA events between its stages; synchronises and
  * stores the stage times in stage_ms: [0] cell sort, [1] spread, [2] forward
  * FFT, [3] convolution, [4] inverse FFT, [5] gather (milliseconds). */
