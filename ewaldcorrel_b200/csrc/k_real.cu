@@ -27,10 +27,10 @@
 // shared memory (x, y in cell units relative to the warp's row, the z
 // fraction and charge as a float4; the z cell relative to the warp's lowest z
 // cell as a separate exact integer; the Cartesian position relative to the
-// warp's first cell), read by broadcast: a reject pass over the 64 computes
-// every lane's distance (Cartesian, against a cutoff widened by 1e-4 of rc^2
-// to cover its rounding, when no image reduction is needed) and builds its
-// bit masks of candidates inside, then each lane evaluates its accepted pairs
+// warp's first cell and its square), read by broadcast: a reject pass over the
+// 64 computes every lane's distance (Cartesian, two candidates per packed
+// instruction, against a cutoff widened to cover its rounding, when no image
+// reduction is needed) and builds its bit masks of candidates inside, then each lane evaluates its accepted pairs
 // one per round (erfc, exp), so the costly part runs on full lanes instead of
 // on the few lanes a candidate happens to be near.  Every pair is visited
 // from both sides, so each point's gradient has one writer and no atomics are
@@ -142,35 +142,59 @@ __device__ __forceinline__ float pair_r2(const RealArgs &A, const RealLane &L, f
   return dxv * dxv + dyv * dyv + dzv * dzv;
 }
 
-// Reject pass over 32 staged candidates: the bit mask of those inside the
-// cutoff (zero separations are dropped later).
-template <bool WRAP>
-__device__ __forceinline__ unsigned real_reject(const RealArgs &A, const RealLane &L, const float4 *__restrict__ cand,
-                                                const float *__restrict__ candz, const float4 *__restrict__ cart) {
+// Staged candidates of the plain reject pass, two at a time for packed FP32
+// arithmetic: (x0, x1, y0, y1) and (z0, z1, |c0|^2, |c1|^2), Cartesian.
+struct RealCart {
+  float4 xy[kRealStage / 2], zn[kRealStage / 2];
+};
+
+typedef unsigned long long f2p;  // two FP32 values, low word first
+__device__ __forceinline__ f2p rpack(float lo, float hi) {
+  f2p r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ f2p rfma(f2p a, f2p b, f2p c) {
+  f2p d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f2p radd(f2p a, f2p b) {
+  f2p d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+// Reject pass over 32 staged candidates: the mask of those inside the cutoff
+// (zero separations are dropped later), candidate k at bit 31 - k.
+__device__ __forceinline__ unsigned real_reject_wrap(const RealArgs &A, const RealLane &L,
+                                                     const float4 *__restrict__ cand,
+                                                     const float *__restrict__ candz) {
   unsigned mask = 0;
-  if (WRAP) {
 #pragma unroll 8
-    for (int k = 0; k < 32; k++) {
-      float dxv, dyv, dzv;
-      const float r2 = pair_r2<WRAP>(A, L, cand[k], candz[k], dxv, dyv, dzv);
-      mask |= (r2 < A.rc2) ? (1u << k) : 0u;
-    }
-  } else {
-    // no image reduction: a plain Cartesian distance against the widened
-    // cutoff; the accepted pairs are tested again from the exact separation.
-    // Eight candidates per byte of the mask, each with a constant bit.
-#pragma unroll 1
-    for (int k0 = 0; k0 < 32; k0 += 8) {
-      unsigned byte = 0;
-#pragma unroll
-      for (int c = 0; c < 8; c++) {
-        const float4 p = cart[k0 + c];
-        const float ddx = p.x - L.px, ddy = p.y - L.py, ddz = p.z - L.pz;
-        const float r2 = ddx * ddx + ddy * ddy + ddz * ddz;
-        byte |= (r2 < A.rc2l) ? (1u << c) : 0u;
-      }
-      mask |= byte << k0;
-    }
+  for (int k = 0; k < 32; k++) {
+    float dxv, dyv, dzv;
+    const float r2 = pair_r2<true>(A, L, cand[k], candz[k], dxv, dyv, dzv);
+    mask |= (r2 < A.rc2) ? (0x80000000u >> k) : 0u;
+  }
+  return mask;
+}
+
+// Without image reduction: |c - p|^2 - thr = |c|^2 - 2 c.p + (|p|^2 - thr) < 0
+// for two candidates at a time; off = |p|^2 - thr and the components of -2 p
+// are the lane's.  The sign bits are shifted into the mask.  The threshold is
+// the cutoff widened past the rounding of this form (see real_chunk); the
+// accepted pairs are tested again from the exact separation.  Four issue
+// slots per candidate instead of ten with differences and a comparison.
+__device__ __forceinline__ unsigned real_reject(const RealCart &cart, int half, f2p px, f2p py, f2p pz, f2p off) {
+  unsigned mask = 0;
+#pragma unroll 8
+  for (int k = 16 * half; k < 16 * half + 16; k++) {
+    const float4 xy = cart.xy[k], zn = cart.zn[k];
+    const f2p t = rfma(rpack(xy.x, xy.y), px,
+                       rfma(rpack(xy.z, xy.w), py, rfma(rpack(zn.x, zn.y), pz, radd(rpack(zn.z, zn.w), off))));
+    mask = __funnelshift_l((unsigned)t, mask, 1);
+    mask = __funnelshift_l((unsigned)(t >> 32), mask, 1);
   }
   return mask;
 }
@@ -182,22 +206,35 @@ __device__ __forceinline__ unsigned real_reject(const RealArgs &A, const RealLan
 // second half holds candidates (warp-uniform).
 template <bool WRAP>
 __device__ __forceinline__ void real_chunk(const RealArgs &A, RealLane &L, const float4 *__restrict__ cand,
-                                           const float *__restrict__ candz, const float4 *__restrict__ cart,
+                                           const float *__restrict__ candz, const RealCart &cart,
                                            const float4 *__restrict__ tab, unsigned live0, unsigned live1,
-                                           bool two) {
-  unsigned m0 = real_reject<WRAP>(A, L, cand, candz, cart) & live0;
-  unsigned m1 = two ? real_reject<WRAP>(A, L, cand + 32, candz + 32, cart + 32) & live1 : 0u;
+                                           bool two, float n2max) {
+  unsigned m0, m1 = 0u;
+  if (WRAP) {
+    m0 = real_reject_wrap(A, L, cand, candz);
+    if (two) m1 = real_reject_wrap(A, L, cand + 32, candz + 32);
+  } else {
+    // five FP32 roundings of terms up to |c|^2 + |p|^2 each: below 6e-7 of
+    // their sum, on top of the 1e-4 of rc^2 that covers the positions' own
+    const float p2 = L.px * L.px + L.py * L.py + L.pz * L.pz;
+    const float off = p2 - (A.rc2l + 1e-6f * (n2max + p2));
+    const f2p px = rpack(-2.f * L.px, -2.f * L.px), py = rpack(-2.f * L.py, -2.f * L.py),
+              pz = rpack(-2.f * L.pz, -2.f * L.pz), of = rpack(off, off);
+    m0 = real_reject(cart, 0, px, py, pz, of);
+    if (two) m1 = real_reject(cart, 1, px, py, pz, of);
+  }
+  m0 &= live0;
+  m1 &= live1;
   const float two_eta_sqrtpi = 1.1283791670955126f * A.eta;  // 2 eta / sqrt(pi)
   const float eta2 = A.eta * A.eta;
   while (m0 | m1) {
-    int k;
-    if (m0) {
-      k = __ffs(m0) - 1;
-      m0 &= m0 - 1;
-    } else {
-      k = 31 + __ffs(m1);
-      m1 &= m1 - 1;
-    }
+    const bool first = m0 != 0u;
+    unsigned m = first ? m0 : m1;
+    const int lead = __clz(m);
+    const int k = lead + (first ? 0 : 32);
+    m ^= 0x80000000u >> lead;
+    m0 = first ? m : 0u;
+    m1 = first ? m1 : m;
     const float4 c = cand[k];
     float dxv, dyv, dzv;
     const float r2 = pair_r2<WRAP>(A, L, c, candz[k], dxv, dyv, dzv);
@@ -205,8 +242,11 @@ __device__ __forceinline__ void real_chunk(const RealArgs &A, RealLane &L, const
     const float ir = rsqrtf(r2);
     const float ex = __expf(-eta2 * r2);  // exp(-x^2), x = eta r (error grows with x^2, where the term is small)
     const float u = A.eta * (r2 * ir) * A.tab_scale;
-    const int ti = min((int)u, kRealTab - 1);
-    const float tt = fminf(u - (float)ti, 1.f);
+    // floor(u) from the low bits of u + 2^23 rounded down: the conversion
+    // instructions share the slow pipe with rsqrt and exp
+    const float uf = fminf(__fadd_rd(u, 8388608.f), 8388608.f + (float)(kRealTab - 1));
+    const int ti = __float_as_int(uf) - 0x4b000000;
+    const float tt = fminf(u - (uf - 8388608.f), 1.f);
     const float4 cf = tab[ti];
     const float erfcx = fmaf(tt, fmaf(tt, fmaf(tt, cf.w, cf.z), cf.y), cf.x);
     const float phi = ex * erfcx * ir;  // erfc(eta r) / r
@@ -238,7 +278,7 @@ __device__ __forceinline__ void real_chunk(const RealArgs &A, RealLane &L, const
 
 // One 32-point group of sorted points per warp at a time, taken from the
 // group counter; writes the group's partials.
-__device__ __forceinline__ void real_group(const RealArgs &A, int grp, float4 *cand, float *candz, float4 *cart,
+__device__ __forceinline__ void real_group(const RealArgs &A, int grp, float4 *cand, float *candz, RealCart &cart,
                                            const float4 *tab) {
   const int lane = threadIdx.x & 31;
   const int i = grp * 32 + lane;
@@ -329,12 +369,13 @@ __device__ __forceinline__ void real_group(const RealArgs &A, int grp, float4 *c
     const int total = __shfl_sync(0xffffffffu, pre, 31);
     pre -= l1 + l2;
     for (int v0 = 0; v0 < total; v0 += kRealStage) {
+     float n2max = 0.f;
 #pragma unroll
      for (int b = 0; b < kRealStage / 32; b++) {
       const int v = v0 + 32 * b + lane;
       float4 cv = make_float4(0.f, 0.f, 0.f, 0.f);  // past the end: masked out below
       float cvz = 0.f;
-      float4 cvp = make_float4(0.f, 0.f, 0.f, 0.f);
+      float3 cvp = make_float3(0.f, 0.f, 0.f);
       // row of stream position v: the last row whose prefix is <= v
       int r = 0;
 #pragma unroll
@@ -355,20 +396,29 @@ __device__ __forceinline__ void real_group(const RealArgs &A, int grp, float4 *c
         cv = make_float4(ro0 + rj.x, ro1 + rj.y, rj.z, rj.w);
         cvz = (float)(cz + sh - zlo);
         const float zc = cvz + rj.z;
-        cvp = make_float4(cv.x * A.ax + cv.y * A.bx + zc * A.cx, cv.y * A.by + zc * A.cy, zc * A.cz, 0.f);
+        cvp = make_float3(cv.x * A.ax + cv.y * A.bx + zc * A.cx, cv.y * A.by + zc * A.cy, zc * A.cz);
       }
       cand[32 * b + lane] = cv;
       candz[32 * b + lane] = cvz;
-      cart[32 * b + lane] = cvp;
+      const float n2 = cvp.x * cvp.x + cvp.y * cvp.y + cvp.z * cvp.z;
+      n2max = fmaxf(n2max, n2);
+      float *xy = reinterpret_cast<float *>(cart.xy + 16 * b) + 4 * (lane >> 1) + (lane & 1);
+      float *zn = reinterpret_cast<float *>(cart.zn + 16 * b) + 4 * (lane >> 1) + (lane & 1);
+      xy[0] = cvp.x;
+      xy[2] = cvp.y;
+      zn[0] = cvp.z;
+      zn[2] = n2;
      }
+      // largest |c|^2 of the batch (nonnegative floats order like their bits)
+      n2max = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(n2max)));
       __syncwarp();
       const int cnt = total - v0;  // candidates left in the stream, > 0
-      const unsigned live0 = act ? (cnt >= 32 ? 0xffffffffu : (1u << cnt) - 1u) : 0u;
-      const unsigned live1 = (act && cnt > 32) ? (cnt >= 64 ? 0xffffffffu : (1u << (cnt - 32)) - 1u) : 0u;
+      const unsigned live0 = act ? (cnt >= 32 ? 0xffffffffu : ~(0xffffffffu >> cnt)) : 0u;
+      const unsigned live1 = (act && cnt > 32) ? (cnt >= 64 ? 0xffffffffu : ~(0xffffffffu >> (cnt - 32))) : 0u;
       if (wrap)
-        real_chunk<true>(A, L, cand, candz, cart, tab, live0, live1, cnt > 32);
+        real_chunk<true>(A, L, cand, candz, cart, tab, live0, live1, cnt > 32, n2max);
       else
-        real_chunk<false>(A, L, cand, candz, cart, tab, live0, live1, cnt > 32);
+        real_chunk<false>(A, L, cand, candz, cart, tab, live0, live1, cnt > 32, n2max);
       __syncwarp();  // every lane has read the batch before the next one is staged
     }
   }
@@ -399,7 +449,7 @@ __device__ __forceinline__ void real_group(const RealArgs &A, int grp, float4 *c
 __global__ void __launch_bounds__(kRealWarps * 32, kRealBlocksPerSM) real_pair_kernel(RealArgs A) {
   __shared__ float4 cand_all[kRealWarps][kRealStage];
   __shared__ float candz_all[kRealWarps][kRealStage];
-  __shared__ float4 cart_all[kRealWarps][kRealStage];
+  __shared__ RealCart cart_all[kRealWarps];
   __shared__ float4 tab[kRealTab];
   for (int k = threadIdx.x; k < kRealTab; k += blockDim.x) tab[k] = A.tab[k];
   __syncthreads();
@@ -416,10 +466,22 @@ __global__ void __launch_bounds__(kRealWarps * 32, kRealBlocksPerSM) real_pair_k
 // out = [E_real, E_self, E_net, vir_real (xx, yy, zz, yx, zx, zy), vir_net
 // (added to each diagonal component)], in de1's virial convention
 // (vir = -W / V with W = sum_pairs q q phi'(r)/r r r^T).
-__global__ void real_finish_kernel(const double *__restrict__ partials, int nblocks, const CellConst *__restrict__ cell,
-                                   double eta, double *__restrict__ out) {
-  __shared__ double tot[9];
-  sum_partials<9>(partials, nblocks, kRealWords, tot);
+// Threads take whole group records in a fixed stride (one warp per component
+// over all records took 19 us for 3072 groups), then a fixed tree.
+constexpr int kFinishThreads = 512;
+__global__ void __launch_bounds__(kFinishThreads) real_finish_kernel(const double *__restrict__ partials, int ngroups,
+                                                                     const CellConst *__restrict__ cell, double eta,
+                                                                     double *__restrict__ out) {
+  __shared__ double red[kFinishThreads / 32][9], tot[9];
+  double acc[9];
+#pragma unroll
+  for (int c = 0; c < 9; c++) acc[c] = 0.0;
+#pragma unroll 2
+  for (int g = threadIdx.x; g < ngroups; g += kFinishThreads)
+#pragma unroll
+    for (int c = 0; c < 9; c++) acc[c] += partials[(long)g * kRealWords + c];
+  block_reduce_n<9>(acc, red, tot);
+  __syncthreads();
   if (threadIdx.x != 0) return;
   const double iV = cell->iV;
   const double pi = 3.14159265358979323846;
@@ -478,7 +540,7 @@ int launch_real_space(const Geom &coarse, const double L[6], int n, const double
     real_pair_kernel<<<blocks, kRealWarps * 32, 0, st>>>(A);
     k += 3;
   }
-  real_finish_kernel<<<1, 9 * 32, 0, st>>>(partials, ngroups, coarse.cell, eta_d, out);
+  real_finish_kernel<<<1, kFinishThreads, 0, st>>>(partials, ngroups, coarse.cell, eta_d, out);
   return k + 1;
 }
 
