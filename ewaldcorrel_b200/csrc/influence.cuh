@@ -311,7 +311,7 @@ __device__ __forceinline__ void block_reduce7(const double (&acc)[7], double (*r
 // Sum of the block partials (warp c sums component c: lanes take blocks in
 // a fixed stride, then a fixed shuffle tree), and the final energy/virial
 // ev = [E, vir_xx, vir_yy, vir_zz, vir_yx, vir_zx, vir_zy] as de1 forms them
-// (sfac.cpp:384-395).  Needs >= 7 warps; raw receives the 7 sums.
+// (sfac.cpp:384-395).  raw receives the 7 sums.
 __device__ __forceinline__ void finish_partials(const double *__restrict__ partials, int nblocks,
                                                 const CellConst *__restrict__ cell, double *__restrict__ raw,
                                                 double *__restrict__ ev) {

@@ -577,8 +577,9 @@ __global__ void __launch_bounds__(512) fft_x2_kernel(int n, int n1, int n2, cons
 // (k1, j2) of line b: (k1*n2 + j2)*B + b.  tw: exp(-2 pi i e / n), e < n.
 
 // y pass: complex lines along y of every x-plane; line l = x*lpp + kz at
-// data[x*pstride + kz + j*es].  With `partials`, CTA 0 first reduces the
-// preceding x pass's energy/virial partials (needs >= 7 warps).
+// data[x*pstride + kz + j*es].  With `partials`, CTA 0 (one more than the
+// lines need) reduces the preceding x pass's energy/virial partials, beside the
+// transform rather than before one of its CTAs' lines.
 template <int SIGN>
 __global__ void __launch_bounds__(512) fft_y2_kernel(int n, int n1, int n2, const float2 *__restrict__ twg,
                                                      float2 *__restrict__ data, long nlines, FastDiv lpp,
@@ -586,13 +587,16 @@ __global__ void __launch_bounds__(512) fft_y2_kernel(int n, int n1, int n2, cons
                                                      const double *__restrict__ partials, int nblocks,
                                                      const CellConst *__restrict__ cell, double *__restrict__ raw,
                                                      double *__restrict__ ev) {
-  if (partials && blockIdx.x == 0) finish_partials(partials, nblocks, cell, raw, ev);
+  if (partials && blockIdx.x == 0) {
+    finish_partials(partials, nblocks, cell, raw, ev);
+    return;
+  }
   extern __shared__ float2 sm[];
   const int B = 1 << lgB;
   float2 *tw = sm, *ex = sm + n;
   for (int i = threadIdx.x; i < n; i += blockDim.x) tw[i] = twg[i];
   const int b = threadIdx.x & (B - 1), t = threadIdx.x >> lgB;
-  const long l = (long)blockIdx.x * B + b;
+  const long l = (long)(blockIdx.x - (partials ? 1 : 0)) * B + b;
   const bool live = l < nlines;
   uint32_t pl = 0, r = 0;
   if (live) lpp.divmod((uint32_t)l, pl, r);
@@ -838,10 +842,9 @@ bool fft_plane_fits(int K1, int K2) {
 long fft_x_blocks_max(int K1, int K2) { return ((long)K1 * (K2 / 2 + 1) + 7) / 8; }
 
 // Shape of a two-level per-axis pass over `nlines` lines of length n:
-// B = 2^lgB lines per CTA (8..32), B*max(n1, n2) threads (at least
-// min_threads, at most 512), B halved while fewer than two CTAs per SM
+// B = 2^lgB lines per CTA (8..32), B*max(n1, n2) threads (at most 512), B halved while fewer than two CTAs per SM
 // (148 SMs) would run.  False when n has no n1 * n2 split.
-static bool lines2_shape(int n, long nlines, int min_threads, int &n1, int &n2, int &lgB, int &threads) {
+static bool lines2_shape(int n, long nlines, int &n1, int &n2, int &lgB, int &threads) {
   if (!rdft::split_line(n, n1, n2)) return false;
   const int m = n1 > n2 ? n1 : n2;
   int B = 8;
@@ -852,7 +855,6 @@ static bool lines2_shape(int n, long nlines, int min_threads, int &n1, int &n2, 
   lgB = 0;
   while ((1 << lgB) < B) lgB++;
   threads = (B * m + 31) / 32 * 32;
-  if (threads < min_threads) threads = min_threads;
   return true;
 }
 
@@ -910,7 +912,7 @@ int fwd_zy(const FftPlan3 &F, const float *real, float2 *cplx, cudaStream_t st) 
   if (zy == ZY_TWO_LEVEL) {
     int n1, n2, lgB, thr;
     launch_z2<true>(K2, F.len[2].tw, const_cast<float *>(real), cplx, (int)nrows, st);
-    lines2_shape(K1, nl, 0, n1, n2, lgB, thr);
+    lines2_shape(K1, nl, n1, n2, lgB, thr);
     const int B = 1 << lgB;
     const size_t smem = (size_t)(K1 + (size_t)B * K1) * sizeof(float2);
     fft_y2_kernel<-1><<<(unsigned)((nl + B - 1) / B), thr, smem, st>>>(K1, n1, n2, F.len[1].tw, cplx, nl,
@@ -949,10 +951,10 @@ int inv_yz(const FftPlan3 &F, float2 *cplx, float *real, const double *partials,
   const long nl = (long)K0 * ldim;
   if (zy == ZY_TWO_LEVEL) {
     int n1, n2, lgB, thr;
-    lines2_shape(K1, nl, partials ? 256 : 0, n1, n2, lgB, thr);
+    lines2_shape(K1, nl, n1, n2, lgB, thr);
     const int B = 1 << lgB;
     const size_t smem = (size_t)(K1 + (size_t)B * K1) * sizeof(float2);
-    fft_y2_kernel<+1><<<(unsigned)((nl + B - 1) / B), thr, smem, st>>>(K1, n1, n2, F.len[1].tw, cplx, nl,
+    fft_y2_kernel<+1><<<(unsigned)((nl + B - 1) / B + (partials ? 1 : 0)), thr, smem, st>>>(K1, n1, n2, F.len[1].tw, cplx, nl,
                                                                        FastDiv(ldim), (long)K1 * ldim, ldim, lgB,
                                                                        partials, nblocks, cell, raw, ev);
     launch_z2<false>(K2, F.len[2].tw, real, cplx, (int)nrows, st);

@@ -581,18 +581,28 @@ void gather_prepare() {
   gather_tile_attr<8, kTileX, kTileY, kTileThreads>();
 }
 
+// Threads per CTA of the thread-per-point kernel: 128 rather than 256 spread
+// the CTAs of mid-size systems more evenly over the SMs (solves of 50k points,
+// order 8: 98.5 -> 94.3 us; 50k, order 4: 61.6 -> 59.6; 64 threads the same,
+// but 4000 points at order 6 55.4 -> 57.5).
+constexpr int kGatherThreads = 128;
+
 template <int P, bool SORTED>
 static int gather_p(const Geom &g, const Spline &S, int n, const double *x, const double *w, const float *grid,
                     double *dx, double *phi, double *cellp, const SortedView &sv, cudaStream_t st) {
-  const int blocks = (n + 255) / 256;
-  if (cellp)
-    gather_kernel<P, true, true, true, SORTED><<<blocks, 256, 0, st>>>(g, S, n, x, w, grid, dx, phi, cellp, sv);
-  else if (dx && phi)
-    gather_kernel<P, true, true, false, SORTED><<<blocks, 256, 0, st>>>(g, S, n, x, w, grid, dx, phi, nullptr, sv);
+  if (cellp) {
+    gather_kernel<P, true, true, true, SORTED>
+        <<<(n + 255) / 256, 256, 0, st>>>(g, S, n, x, w, grid, dx, phi, cellp, sv);
+    return 1;
+  }
+  constexpr int threads = kGatherThreads;
+  const int blocks = (n + threads - 1) / threads;
+  if (dx && phi)
+    gather_kernel<P, true, true, false, SORTED><<<blocks, threads, 0, st>>>(g, S, n, x, w, grid, dx, phi, nullptr, sv);
   else if (dx)
-    gather_kernel<P, true, false, false, SORTED><<<blocks, 256, 0, st>>>(g, S, n, x, w, grid, dx, phi, nullptr, sv);
+    gather_kernel<P, true, false, false, SORTED><<<blocks, threads, 0, st>>>(g, S, n, x, w, grid, dx, phi, nullptr, sv);
   else if (phi)
-    gather_kernel<P, false, true, false, SORTED><<<blocks, 256, 0, st>>>(g, S, n, x, w, grid, dx, phi, nullptr, sv);
+    gather_kernel<P, false, true, false, SORTED><<<blocks, threads, 0, st>>>(g, S, n, x, w, grid, dx, phi, nullptr, sv);
   else return 0;
   return 1;
 }

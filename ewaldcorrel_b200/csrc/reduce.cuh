@@ -31,14 +31,14 @@ __device__ __forceinline__ void block_reduce_n(const double (&acc)[NC], double (
   }
 }
 
-// Sum over nblocks partial vectors (stride `stride` doubles) of component
-// c = warp index: lanes take blocks in a fixed stride, then a fixed tree.
-// Needs >= NC warps; the totals land in tot[0..NC).
+// Sum over nblocks partial vectors (stride `stride` doubles) of component c,
+// by warp c modulo the warps of the block: lanes take blocks in a fixed
+// stride, then a fixed tree.  The totals land in tot[0..NC).
 template <int NC>
 __device__ __forceinline__ void sum_partials(const double *__restrict__ partials, int nblocks, int stride,
                                              double *tot) {
-  const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (c < NC) {
+  const int lane = threadIdx.x & 31;
+  for (int c = threadIdx.x >> 5; c < NC; c += blockDim.x >> 5) {
     double v = 0.0;
     for (int b = lane; b < nblocks; b += 32) v += partials[(long)b * stride + c];
     v = warp_sum(v);
