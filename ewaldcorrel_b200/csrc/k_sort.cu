@@ -284,11 +284,15 @@ static BucketMap bucket_map(const Geom &g, int zshift) {
 
 // Slots of the buckets (the sort in two passes): slot s < ns of bucket b
 // holds the (key, index) of its s-th arrival; later arrivals form a chain
-// from spill[b] over next[] (index + 1, 0: the end).
+// from spill[b] over next[] (index + 1, 0: the end).  The first four slots of
+// all buckets come first, then the next four, and so on: an ordinary system
+// touches little beyond the first quarter of the space.
 struct Slots {
   uint2 *at;
   int ns;
   uint32_t *spill, *next;
+  uint32_t nb;
+  __device__ __forceinline__ uint2 *quad(uint32_t b, int s) const { return at + 4 * ((size_t)(s >> 2) * nb + b); }
 };
 
 // head/tail (may be null): see the word layout above; ht_h = H.  tsum (may be
@@ -320,7 +324,7 @@ __global__ void __launch_bounds__(256) key_count_kernel(Geom g, int n, const dou
       const uint32_t s = atomicAdd(&count[b], 1u);
       slot[a] = s;
       if (sl.at) {
-        if (s < (uint32_t)sl.ns) sl.at[(size_t)b * sl.ns + s] = make_uint2(key, (uint32_t)a);
+        if (s < (uint32_t)sl.ns) sl.quad(b, (int)s)[s & 3] = make_uint2(key, (uint32_t)a);
         else sl.next[a] = atomicExch(&sl.spill[b], (uint32_t)a + 1u);
       }
       if (head) {
@@ -576,7 +580,6 @@ __global__ void __launch_bounds__(256) cell_place_kernel(int n, const uint32_t *
     const float4 r = rec[a];
     b = bm(key);
     if (SPME_IN(b, bm.nb, CK_SORT_BUCKET)) {
-      const uint2 *at = sl.at + (size_t)b * sl.ns;
       const int lo = cs[b], c = cs[b + 1] - lo;
       if (c > kBigCell) {
         const int s = (int)slot[a];
@@ -590,8 +593,9 @@ __global__ void __launch_bounds__(256) cell_place_kernel(int n, const uint32_t *
         int rank = 0;
         if (c > 1) {
           const int m = min(c, sl.ns);
-          for (int j = 0; j < m; j += 4) {  // ns is a multiple of 4: whole 32-byte reads stay in the bucket's slots
-            const uint4 p = *reinterpret_cast<const uint4 *>(at + j), q = *reinterpret_cast<const uint4 *>(at + j + 2);
+          for (int j = 0; j < m; j += 4) {
+            const uint4 *at = reinterpret_cast<const uint4 *>(sl.quad(b, j));
+            const uint4 p = at[0], q = at[1];
             rank += pair_less(p.x, p.y, key, (uint32_t)a) ? 1 : 0;
             rank += j + 1 < m && pair_less(p.z, p.w, key, (uint32_t)a) ? 1 : 0;
             rank += j + 2 < m && pair_less(q.x, q.y, key, (uint32_t)a) ? 1 : 0;
@@ -736,11 +740,10 @@ __global__ void __launch_bounds__(kSmallThreads) cell_sort_small_kernel(
 
 // The sort by slots takes the place of the scatter and fix-up while a bucket
 // holds few enough atoms for its slots (at a mean of half of them less three,
-// 5 of 16, about one bucket in 70,000 spills) and while the slots, written
-// and read in pieces of 32 bytes, stay small in L2: a solve of 98k atoms on
-// 96^3 (3.5 MB of slots) took 71.9 us against 73.8, 200k on 128^3 132.9 / 134.9,
-// 400k on 160^3 (16 MB) 247.9 / 249.2, but 600k on 192^3 (28 MB) 332.6 / 325.9
-// and 1M on 256^3 (67 MB) 605 / 592.
+// 5 of 16, about one bucket in 70,000 spills) and while they stay small in
+// L2: a solve of 98k atoms on 96^3 (3.5 MB of slots) took 67.8 us against
+// 70.8, 200k on 128^3 126.6 / 129.1, 400k on 160^3 (16 MB) 230.6 / 238.7, but
+// 600k on 192^3 (28 MB) 308.4 / 303.5 and 1M on 256^3 (67 MB) 549.6 / 543.9.
 constexpr double kSlotsMaxBytes = 1 << 24;
 static bool use_slots(const Geom &g, int n, const SortBuffers &b, int zshift) {
   const double mean = (double)n * (double)(1 << zshift) / ((double)g.K0 * g.K1 * g.K2);
@@ -776,7 +779,7 @@ int launch_cell_sort(const Geom &g, int n, const double *x, const double *w, Sor
   const bool slots = use_slots(g, n, b, zshift);
   // tile sums taken while counting, while they are few (more: one pass over the counts)
   const bool count_tiles = ntiles > 1 && ntiles <= kCountTiles && n > 0;
-  const Slots sl{slots ? b.slots : nullptr, b.nslot, spill, b.next};
+  const Slots sl{slots ? b.slots : nullptr, b.nslot, spill, b.next, (uint32_t)nb};
   cudaMemsetAsync(count, 0, sizeof(uint32_t) * (3 * nb + 1 + ntiles + (slots ? nb : 0)), st);
   int launches = 0;
   if (n > 0) {
