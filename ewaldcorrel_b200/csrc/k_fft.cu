@@ -265,8 +265,6 @@ __global__ void __launch_bounds__(512) fft_plane_inv_kernel(FftLen Ly, FftLen Lz
 //                   en() and de1() return the same energy bit for bit.
 // Energy/virial sums are FP64, reduced per CTA in a fixed order (lane tree,
 // then warps in order) into partials[blockIdx.x].
-enum { XM_FWD_DECONV = 0, XM_CONV_INV = 1, XM_FWD_CONV_INV = 2, XM_EN = 3 };
-
 template <int MODE>
 __global__ void __launch_bounds__(256) fft_x_kernel(FftLen L, Geom g, Influence inf, const double *__restrict__ iB0,
                                                     const double *__restrict__ iB1, const double *__restrict__ iB2,
@@ -803,6 +801,7 @@ static void fft_shape(int n, long nlines, int &B, int &bufsz, size_t &smem) {
 }
 
 void fft_prepare_kernels() {
+  fft_groups_prepare();
   const int lim = 200 * 1024;
   cudaFuncSetAttribute((const void *)fft_z_r2c_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute((const void *)fft_z_c2r_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
@@ -883,22 +882,38 @@ static void launch_z2(int n, const float2 *tw, float *real, float2 *cplx, int nr
 // Which z/y implementation a plan uses: the fused plane kernels (an x-plane
 // in shared memory), the two-level per-axis passes, or the Stockham
 // per-axis passes (any length).
-enum { ZY_PLANE = 1, ZY_TWO_LEVEL = 2, ZY_STOCKHAM = 3 };
-static int zy_choice(const FftPlan3 &F) {
+// Groups take the place of the plane and per-axis Stockham passes (the same
+// stages, and the same pairs of rows: within each x-plane where the plane fits;
+// so the same bits) wherever both lengths have them.
+enum { ZY_PLANE = 1, ZY_TWO_LEVEL = 2, ZY_STOCKHAM = 3, ZY_GROUPS = 4 };
+static int zy_choice(const FftPlan3 &F, FftGroups &Gy, FftGroups &Gz, bool &plane) {
   const int K1 = F.len[1].n, K2 = F.len[2].n;
   int sz, a, b;
-  const bool plane = plane_smem(K1, K2, sz) <= kPlaneSmemMax;
+  plane = plane_smem(K1, K2, sz) <= kPlaneSmemMax;
   const bool two = rdft::split_line(K1, a, b) && rdft::split_line(K2, a, b);
   if (F.zy_mode == ZY_PLANE && plane) return ZY_PLANE;
   if (F.zy_mode == ZY_STOCKHAM) return ZY_STOCKHAM;
   if (two) return ZY_TWO_LEVEL;
+  if (fft_group_split(F.len[1], Gy) && fft_group_split(F.len[2], Gz)) return ZY_GROUPS;
   return plane ? ZY_PLANE : ZY_STOCKHAM;
+}
+
+static Geom zy_geom(const FftPlan3 &F, const CellConst *cell) {
+  Geom g{};
+  g.K0 = F.len[0].n;
+  g.K1 = F.len[1].n;
+  g.K2 = F.len[2].n;
+  g.ldim = g.K2 / 2 + 1;
+  g.cell = cell;
+  return g;
 }
 
 // Forward z (r2c) and y transforms.
 int fwd_zy(const FftPlan3 &F, const float *real, float2 *cplx, cudaStream_t st) {
   const int K0 = F.len[0].n, K1 = F.len[1].n, K2 = F.len[2].n, ldim = K2 / 2 + 1;
-  const int zy = zy_choice(F);
+  FftGroups Gy, Gz;
+  bool plane;
+  const int zy = zy_choice(F, Gy, Gz, plane);
   if (zy == ZY_PLANE) {
     int sz;
     const size_t psm = plane_smem(K1, K2, sz);
@@ -920,6 +935,11 @@ int fwd_zy(const FftPlan3 &F, const float *real, float2 *cplx, cudaStream_t st) 
                                                                        nullptr, 0, nullptr, nullptr, nullptr);
     return 2;
   }
+  if (zy == ZY_GROUPS) {
+    launch_groups_z(Gz, true, const_cast<float *>(real), cplx, plane ? K0 : 1, plane ? K1 : (int)nrows, st);
+    launch_groups_y(Gy, true, zy_geom(F, nullptr), cplx, nullptr, 0, nullptr, nullptr, st);
+    return 2;
+  }
   int B, bufsz;
   size_t smem;
   fft_shape(K2, (nrows + 1) / 2, B, bufsz, smem);
@@ -937,7 +957,9 @@ int fwd_zy(const FftPlan3 &F, const float *real, float2 *cplx, cudaStream_t st) 
 int inv_yz(const FftPlan3 &F, float2 *cplx, float *real, const double *partials, int nblocks,
            const CellConst *cell, double *raw, double *ev, cudaStream_t st) {
   const int K0 = F.len[0].n, K1 = F.len[1].n, K2 = F.len[2].n, ldim = K2 / 2 + 1;
-  const int zy = zy_choice(F);
+  FftGroups Gy, Gz;
+  bool plane;
+  const int zy = zy_choice(F, Gy, Gz, plane);
   if (zy == ZY_PLANE) {
     int sz;
     const size_t psm = plane_smem(K1, K2, sz);
@@ -958,6 +980,11 @@ int inv_yz(const FftPlan3 &F, float2 *cplx, float *real, const double *partials,
                                                                        FastDiv(ldim), (long)K1 * ldim, ldim, lgB,
                                                                        partials, nblocks, cell, raw, ev);
     launch_z2<false>(K2, F.len[2].tw, real, cplx, (int)nrows, st);
+    return 2;
+  }
+  if (zy == ZY_GROUPS) {
+    launch_groups_y(Gy, false, zy_geom(F, cell), cplx, partials, nblocks, raw, ev, st);
+    launch_groups_z(Gz, false, real, cplx, plane ? K0 : 1, plane ? K1 : (int)nrows, st);
     return 2;
   }
   int k = 0;
@@ -1035,6 +1062,11 @@ static int x_pass(const FftPlan3 &F, const Geom &g, const Influence &inf, const 
     if (MODE == XM_FWD_DECONV || inf.mode == 1) go(std::integral_constant<int, 1>{});
     else if (inf.mode == 4) go(std::integral_constant<int, 4>{});
     else go(std::integral_constant<int, 2>{});
+    return 1;
+  }
+  FftGroups G;
+  if (F.x_lines == 0 && fft_group_split(F.len[0], G)) {
+    launch_groups_x(G, MODE, g, inf, iB0, iB1, iB2, cplx, partials, nblocks, st);
     return 1;
   }
   int B = x_lines_per_cta(F, n, nl);

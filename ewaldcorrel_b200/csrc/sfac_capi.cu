@@ -1276,7 +1276,8 @@ int sfac_check_take(unsigned long long *word) {
   if (cudaDeviceSynchronize() != cudaSuccess) return -1;
   unsigned long long (*const take[])() = {spme::check_take_sort,  spme::check_take_spread,
                                           spme::check_take_gather, spme::check_take_fft,
-                                          spme::check_take_serve,  spme::check_take_capi};
+                                          spme::check_take_serve,  spme::check_take_capi,
+                                          spme::check_take_fft_groups};
   int first = 0;
   for (int m = 0; m < (int)(sizeof(take) / sizeof(take[0])); m++) {
     const unsigned long long v = take[m]();

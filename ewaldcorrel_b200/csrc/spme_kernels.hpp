@@ -20,6 +20,7 @@ unsigned long long check_take_sort();
 unsigned long long check_take_spread();
 unsigned long long check_take_gather();
 unsigned long long check_take_fft();
+unsigned long long check_take_fft_groups();
 unsigned long long check_take_serve();
 unsigned long long check_take_capi();
 
@@ -75,6 +76,14 @@ struct DeconvArgs {
   const double *iB0, *iB1, *iB2;  // null: no moduli division
   int ldim;
 };
+// A line as two groups of Stockham stages in registers (k_fft_groups.cu):
+// n = n1 n2, the groups' ids, the table of FftLen.
+struct FftGroups {
+  int n, n1, n2, g1, g2;
+  const float2 *tw;
+};
+// Modes of the x pass (k_fft.cu).
+enum { XM_FWD_DECONV = 0, XM_CONV_INV = 1, XM_FWD_CONV_INV = 2, XM_EN = 3 };
 int fft_make_len(FftLen &L, int n, float2 *tw_dev, cudaStream_t st);
 void fft_prepare_kernels();  // sets shared-memory limits once (before any graph capture)
 bool fft_plane_fits(int K1, int K2);
@@ -105,6 +114,17 @@ int inv_yz(const FftPlan3 &F, float2 *cplx, float *real, const double *partials,
 int launch_fft_conv_solve(const FftPlan3 &F, const Geom &g, const Influence &inf, const double *iB0,
                           const double *iB1, const double *iB2, const float *real_in, float2 *cplx,
                           float *real_out, double *partials, double *raw, double *ev, cudaStream_t st);
+
+// ---- FFT passes by groups of stages (k_fft_groups.cu) ----
+bool fft_group_split(const FftLen &L, FftGroups &G);
+void fft_groups_prepare();  // sets shared-memory limits once (before any graph capture)
+// planes x rpp rows, paired within each plane
+void launch_groups_z(const FftGroups &F, bool forward, float *real, float2 *cplx, int planes, int rpp, cudaStream_t st);
+void launch_groups_y(const FftGroups &F, bool forward, const Geom &g, float2 *cplx, const double *partials, int nblocks,
+                     double *raw, double *ev, cudaStream_t st);
+void launch_groups_x(const FftGroups &F, int mode, const Geom &g, const Influence &inf, const double *iB0,
+                     const double *iB1, const double *iB2, float2 *cplx, double *partials, int &nblocks,
+                     cudaStream_t st);
 
 // ---- moduli, influence function, convolution (k_conv.cu) ----
 // M_order(j), j = 0..order-1: the B-spline at the integer nodes (FP64).

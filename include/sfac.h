@@ -329,7 +329,7 @@ int sfac_debug_fail_alloc(int nth);
  * sfac_check_take: after a device synchronize, reads and clears every
  *   module's word; returns 0 if no check failed since the last call, else
  *   the first failing module (1 sort, 2 spread, 3 gather, 4 FFT and
- *   convolution, 5 serving, 6 C API) with its word in *word (may be NULL);
+ *   convolution, 5 serving, 6 C API, 7 FFT by groups of stages) with its word in *word (may be NULL);
  *   -1 if the device reports an error.
  * sfac_check_selftest: runs one check that must fail (its store stays inside
  *   its buffer either way) and returns 0 if the word came back as expected,
