@@ -88,7 +88,8 @@ struct Handle {
   RowImg *d_rows = nullptr;  // K0*K1 row image tables (device Ewald mode)
   double *d_partials = nullptr, *d_red = nullptr, *d_ev = nullptr;
   int cap = 0;
-  double *d_x = nullptr, *d_w = nullptr;
+  double *d_x = nullptr, *d_w = nullptr;  // d_w: the last quarter of d_x's allocation
+  uint32_t *d_words = nullptr;            // the sort's word buffers, back to back
   SortBuffers sb{};
   int gcap = 0;
   double *d_gx = nullptr, *d_gw = nullptr, *d_gout = nullptr;
@@ -281,35 +282,28 @@ bool ensure_real(Handle *h, int n, long ncell) {
 
 void free_atoms(Handle *h) {
   dfree(h->d_x);
-  dfree(h->d_w);
-  for (int i = 0; i < 2; i++) {
-    dfree(h->sb.keys[i]);
-    dfree(h->sb.vals[i]);
-  }
-  dfree(h->sb.tmp);
-  dfree(h->sb.tkeys);
-  dfree(h->sb.next);
+  dfree(h->d_words);
   dfree(h->sb.rec);
-  dfree(h->sb.rec_sorted);
-  dfree(h->sb.hist);
+  h->d_w = nullptr;
   h->cap = 0;
 }
 
+// Atom buffers in three allocations (one each made a handle's first pass wait
+// for eleven cudaMalloc calls).
 bool ensure_atoms(Handle *h, int n) {
   if (n <= h->cap) return true;
   free_atoms(h);
-  const int cap = n + n / 2 + 64;
-  bool ok = dalloc(h, &h->d_x, 3 * (size_t)cap) && dalloc(h, &h->d_w, cap);
-  for (int i = 0; i < 2; i++) ok = ok && dalloc(h, &h->sb.keys[i], cap) && dalloc(h, &h->sb.vals[i], cap);
-  ok = ok && dalloc(h, &h->sb.tmp, cap) && dalloc(h, &h->sb.tkeys, cap) && dalloc(h, &h->sb.next, cap) &&
-       dalloc(h, &h->sb.rec, cap) &&
-       dalloc(h, &h->sb.rec_sorted, cap) &&
-       dalloc(h, &h->sb.hist, cap);
-  if (!ok) {
+  const size_t cap = ((size_t)n + n / 2 + 64 + 3) / 4 * 4;
+  if (!(dalloc(h, &h->d_x, 4 * cap) && dalloc(h, &h->d_words, 8 * cap) && dalloc(h, &h->sb.rec, 2 * cap))) {
     free_atoms(h);
     return false;
   }
-  h->cap = cap;
+  h->d_w = h->d_x + 3 * cap;
+  h->sb.rec_sorted = h->sb.rec + cap;
+  uint32_t **words[8] = {&h->sb.keys[0], &h->sb.keys[1], &h->sb.vals[0], &h->sb.vals[1],
+                         &h->sb.tkeys,   &h->sb.tmp,     &h->sb.next,    &h->sb.hist};
+  for (int i = 0; i < 8; i++) *words[i] = h->d_words + i * cap;
+  h->cap = (int)cap;
   h->version++;  // buffers moved: cached graphs are stale
   return true;
 }
