@@ -83,7 +83,8 @@ struct SpStage {
   f2r zq[32][C::ZQE];  // (w(zs + 2m), w(zs + 2m + 1)): z taps from the even zs <= rz, zero off the stencil
   __align__(16) f2r wxl[32][5];  // x weights of columns (2 lx, 2 lx + 1), lx = 0..3 (row padded to 5 pairs)
   __align__(16) float wyl[32][9]; // y weights of rows 0..7 (padded to 9: the staging stores spread over the banks)
-  int cnt[64];         // atoms per window case in the chunk, then the case starts
+  int cnt[64];         // atoms per window case in the chunk
+  __align__(4) uint8_t first[64];  // the cases' first rows (at most 32)
 };
 constexpr int kRowMap = 512;
 static_assert(SpCfg<8>::NR <= 256, "halo rows fit a byte");
@@ -125,11 +126,15 @@ __device__ __forceinline__ void sp_taps(f2r (&acc)[2][SP_TZ / 2], f2r d0, f2r d1
 
 // The walk over one staged chunk, window case by window case: case C (all
 // compile-time, so every accumulator index is fixed) adds the staged rows
-// [start[C], start[C + 1]); a case absent from the chunk costs one test.
+// [first[C], first[C + 1]); a case absent from the chunk costs one test.  The
+// first rows are bytes, read four cases at a time (w): a load per case put
+// some 20 shared-memory latencies in series into every chunk.
 template <int P, int C>
-__device__ __forceinline__ void sp_walk(f2r (&acc)[2][SP_TZ / 2], const SpStage<P> &st, int lx, int ly, int k) {
+__device__ __forceinline__ void sp_walk(f2r (&acc)[2][SP_TZ / 2], const SpStage<P> &st, int lx, int ly, int k,
+                                        uint32_t w) {
   if constexpr (C < SpCfg<P>::NC) {
-    const int e = st.cnt[C + 1];
+    if constexpr (C == 0 || (C + 1) % 4 == 0) w = reinterpret_cast<const uint32_t *>(st.first)[(C + 1) / 4];
+    const int e = (int)((w >> (8 * ((C + 1) % 4))) & 0xffu);
 #pragma unroll 1
     for (; k < e; k++) {
       const float2 xp = *reinterpret_cast<const float2 *>(&st.wxl[k][lx]);
@@ -145,7 +150,7 @@ __device__ __forceinline__ void sp_walk(f2r (&acc)[2][SP_TZ / 2], const SpStage<
       }
       sp_taps<P, C>(acc, d0, d1, zq);
     }
-    sp_walk<P, C + 1>(acc, st, lx, ly, k);
+    sp_walk<P, C + 1>(acc, st, lx, ly, k, w);
   }
 }
 
@@ -159,8 +164,16 @@ __device__ __forceinline__ void group_sync(int group) {
   }
 }
 
-// First index in [lo, hi) whose key is >= k (keys sorted).
+// First index in [lo, hi) whose key is >= k (keys sorted).  Up to four keys
+// (most buckets) are read together and counted: one load latency, not two or
+// three in series.
 __device__ __forceinline__ int keys_lower_bound(const uint32_t *__restrict__ keys, int lo, int hi, uint32_t k) {
+  if (hi - lo <= 4) {
+    int c = 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) c += (lo + i < hi && __ldg(keys + lo + i) < k) ? 1 : 0;
+    return lo + c;
+  }
   while (lo < hi) {
     const int m = (lo + hi) >> 1;
     if (__ldg(keys + m) < k) lo = m + 1; else hi = m;
@@ -248,17 +261,24 @@ __global__ void __launch_bounds__(SP_WARPS * 32, SP_MIN_CTAS) spread_kernel(SpAr
     }
     group_sync<NS>(group);
     if (member == 0) {
-      int running = 0;
-      for (int c = 0; c < NR; c += 32) {
-        const int r = c + lane;
-        int v = (r < NR) ? gr.pref[r + 1] : 0;
+      // all rows' scans side by side: their shuffles overlap
+      constexpr int NW = (NR + 31) / 32;
+      int v[NW];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int u = __shfl_up_sync(0xffffffffu, v, o);
-          if (lane >= o) v += u;
+      for (int c = 0; c < NW; c++) v[c] = (32 * c + lane < NR) ? gr.pref[32 * c + lane + 1] : 0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+        for (int c = 0; c < NW; c++) {
+          const int u = __shfl_up_sync(0xffffffffu, v[c], o);
+          if (lane >= o) v[c] += u;
         }
-        if (r < NR) gr.pref[r + 1] = running + v;
-        running += __shfl_sync(0xffffffffu, v, 31);
+      }
+      int running = 0;
+#pragma unroll
+      for (int c = 0; c < NW; c++) {
+        if (32 * c + lane < NR) gr.pref[32 * c + lane + 1] = running + v[c];
+        running += __shfl_sync(0xffffffffu, v[c], 31);
       }
       if (lane == 0) gr.pref[0] = 0;
     }
@@ -318,9 +338,7 @@ __global__ void __launch_bounds__(SP_WARPS * 32, SP_MIN_CTAS) spread_kernel(SpAr
           const int u = __shfl_up_sync(0xffffffffu, incl, o);
           if (lane >= o) incl += u;
         }
-        __syncwarp();
-        st.cnt[2 * lane] = incl - e0 - e1;
-        st.cnt[2 * lane + 1] = incl - e1;
+        reinterpret_cast<uint16_t *>(st.first)[lane] = (uint16_t)((incl - e0 - e1) | (incl - e1) << 8);
       }
       // zero the chunk's x/y weight rows with contiguous stores of the whole warp
       {
@@ -337,7 +355,7 @@ __global__ void __launch_bounds__(SP_WARPS * 32, SP_MIN_CTAS) spread_kernel(SpAr
       }
       __syncwarp();
       if (valid) {
-        int row = st.cnt[mycase] + __popc(peers & ((1u << lane) - 1u));
+        int row = st.first[mycase] + __popc(peers & ((1u << lane) - 1u));
         if (!SPME_IN(row, 32, CK_SPREAD_ROW)) row = 0;
         // tap i of each axis: the weight of point first + i, M(f + P - 1 - i);
         // the brick's column c = i + rx - (P - 1) takes tap i (zero elsewhere)
@@ -369,7 +387,7 @@ __global__ void __launch_bounds__(SP_WARPS * 32, SP_MIN_CTAS) spread_kernel(SpAr
               make_ulonglong2(pack2(zv[4 * v], zv[4 * v + 1]), pack2(zv[4 * v + 2], zv[4 * v + 3]));
       }
       __syncwarp();
-      sp_walk<P, 0>(acc, st, lx, ly, 0);
+      sp_walk<P, 0>(acc, st, lx, ly, 0, 0u);
       __syncwarp();  // the next chunk's staging overwrites these atoms
     }
     ezs += len;
