@@ -24,7 +24,8 @@ SPME_CHECK_READER(fft)
 // CTA handles 2B real rows (B complex lines); row pitch K2 (real) / ldim.
 __global__ void __launch_bounds__(256) fft_z_r2c_kernel(FftLen L, int nrows, const float *__restrict__ rin,
                                                         float2 *__restrict__ cout, int ldim, int B,
-                                                        int bufsz, FastDiv Bd) {
+                                                        int bufsz, FastDiv Bd, ZeroWords zw) {
+  zero_words(zw);
   extern __shared__ float2 sm[];
   const int n = L.n, P = B + 1;
   float2 *tw = sm, *b0 = sm + n, *b1 = b0 + bufsz;
@@ -142,7 +143,8 @@ __global__ void __launch_bounds__(256) fft_strided_kernel(FftLen L, long nlines,
 // warp-synchronous over a warp's own columns (dz / dy: columns per warp).
 __global__ void __launch_bounds__(512) fft_plane_fwd_kernel(FftLen Ly, FftLen Lz, const float *__restrict__ rin,
                                                             float2 *__restrict__ cout, int sz, FastDiv dz, FastDiv dy,
-                                                            FastDiv dK2, FastDiv dldim) {
+                                                            FastDiv dK2, FastDiv dldim, ZeroWords zw) {
+  zero_words(zw);
   extern __shared__ float2 sm[];
   const int K1 = Ly.n, K2 = Lz.n, ldim = K2 / 2 + 1;
   float2 *twy = sm, *twz = twy + K1, *A = twz + K2, *Bf = A + sz;
@@ -646,7 +648,9 @@ template <int G>
 __global__ void __launch_bounds__(32 * kZWarps) fft_z2_r2c_kernel(int n, int n1, int n2,
                                                                   const float2 *__restrict__ twg,
                                                                   const float *__restrict__ rin,
-                                                                  float2 *__restrict__ cout, int nrows) {
+                                                                  float2 *__restrict__ cout, int nrows,
+                                                                  ZeroWords zw) {
+  zero_words(zw);
   extern __shared__ float2 sm[];
   constexpr int LW = 32 / G;  // lines per warp
   const int ldim = n / 2 + 1, exn = n1 * (n2 + 1);
@@ -860,7 +864,8 @@ static bool lines2_shape(int n, long nlines, int &n1, int &n2, int &lgB, int &th
 // Two-level z pass over nrows rows of length n: groups of 8 or 16 lanes, and
 // fewer warps per CTA while the SMs would not all get one.
 template <bool FWD>
-static void launch_z2(int n, const float2 *tw, float *real, float2 *cplx, int nrows, cudaStream_t st) {
+static void launch_z2(int n, const float2 *tw, float *real, float2 *cplx, int nrows, const ZeroWords &zw,
+                      cudaStream_t st) {
   int n1, n2;
   rdft::split_line(n, n1, n2);
   const bool small = n1 <= 8;  // n2 <= n1
@@ -871,8 +876,8 @@ static void launch_z2(int n, const float2 *tw, float *real, float2 *cplx, int nr
   const size_t smem = (size_t)(n + wpc * lw * n1 * (n2 + 1)) * sizeof(float2);
   const unsigned blocks = (unsigned)((warps + wpc - 1) / wpc);
   if (FWD) {
-    if (small) fft_z2_r2c_kernel<8><<<blocks, 32 * wpc, smem, st>>>(n, n1, n2, tw, real, cplx, nrows);
-    else fft_z2_r2c_kernel<16><<<blocks, 32 * wpc, smem, st>>>(n, n1, n2, tw, real, cplx, nrows);
+    if (small) fft_z2_r2c_kernel<8><<<blocks, 32 * wpc, smem, st>>>(n, n1, n2, tw, real, cplx, nrows, zw);
+    else fft_z2_r2c_kernel<16><<<blocks, 32 * wpc, smem, st>>>(n, n1, n2, tw, real, cplx, nrows, zw);
   } else {
     if (small) fft_z2_c2r_kernel<8><<<blocks, 32 * wpc, smem, st>>>(n, n1, n2, tw, cplx, real, nrows);
     else fft_z2_c2r_kernel<16><<<blocks, 32 * wpc, smem, st>>>(n, n1, n2, tw, cplx, real, nrows);
@@ -908,8 +913,8 @@ static Geom zy_geom(const FftPlan3 &F, const CellConst *cell) {
   return g;
 }
 
-// Forward z (r2c) and y transforms.
-int fwd_zy(const FftPlan3 &F, const float *real, float2 *cplx, cudaStream_t st) {
+// Forward z (r2c) and y transforms; the first kernel also zeroes zw.
+int fwd_zy(const FftPlan3 &F, const float *real, float2 *cplx, const ZeroWords &zw, cudaStream_t st) {
   const int K0 = F.len[0].n, K1 = F.len[1].n, K2 = F.len[2].n, ldim = K2 / 2 + 1;
   FftGroups Gy, Gz;
   bool plane;
@@ -919,14 +924,14 @@ int fwd_zy(const FftPlan3 &F, const float *real, float2 *cplx, cudaStream_t st) 
     const size_t psm = plane_smem(K1, K2, sz);
     const int nb1 = (K1 + 1) / 2;
     fft_plane_fwd_kernel<<<K0, 512, psm, st>>>(F.len[1], F.len[2], real, cplx, sz, FastDiv((nb1 + 15) / 16),
-                                               FastDiv((ldim + 15) / 16), FastDiv(K2), FastDiv(ldim));
+                                               FastDiv((ldim + 15) / 16), FastDiv(K2), FastDiv(ldim), zw);
     return 1;
   }
   const long nrows = (long)K0 * K1;
   const long nl = (long)K0 * ldim;
   if (zy == ZY_TWO_LEVEL) {
     int n1, n2, lgB, thr;
-    launch_z2<true>(K2, F.len[2].tw, const_cast<float *>(real), cplx, (int)nrows, st);
+    launch_z2<true>(K2, F.len[2].tw, const_cast<float *>(real), cplx, (int)nrows, zw, st);
     lines2_shape(K1, nl, n1, n2, lgB, thr);
     const int B = 1 << lgB;
     const size_t smem = (size_t)(K1 + (size_t)B * K1) * sizeof(float2);
@@ -936,7 +941,7 @@ int fwd_zy(const FftPlan3 &F, const float *real, float2 *cplx, cudaStream_t st) 
     return 2;
   }
   if (zy == ZY_GROUPS) {
-    launch_groups_z(Gz, true, const_cast<float *>(real), cplx, plane ? K0 : 1, plane ? K1 : (int)nrows, st);
+    launch_groups_z(Gz, true, const_cast<float *>(real), cplx, plane ? K0 : 1, plane ? K1 : (int)nrows, zw, st);
     launch_groups_y(Gy, true, zy_geom(F, nullptr), cplx, nullptr, 0, nullptr, nullptr, st);
     return 2;
   }
@@ -944,7 +949,7 @@ int fwd_zy(const FftPlan3 &F, const float *real, float2 *cplx, cudaStream_t st) 
   size_t smem;
   fft_shape(K2, (nrows + 1) / 2, B, bufsz, smem);
   fft_z_r2c_kernel<<<(unsigned)((nrows + 2 * B - 1) / (2 * B)), 256, smem, st>>>(F.len[2], (int)nrows, real, cplx,
-                                                                                 ldim, B, bufsz, FastDiv(B));
+                                                                                 ldim, B, bufsz, FastDiv(B), zw);
   fft_shape(K1, nl, B, bufsz, smem);
   DeconvArgs none{};
   fft_strided_kernel<-1><<<(int)((nl + B - 1) / B), 256, smem, st>>>(F.len[1], nl, ldim, (long)K1 * ldim, ldim,
@@ -979,12 +984,12 @@ int inv_yz(const FftPlan3 &F, float2 *cplx, float *real, const double *partials,
     fft_y2_kernel<+1><<<(unsigned)((nl + B - 1) / B + (partials ? 1 : 0)), thr, smem, st>>>(K1, n1, n2, F.len[1].tw, cplx, nl,
                                                                        FastDiv(ldim), (long)K1 * ldim, ldim, lgB,
                                                                        partials, nblocks, cell, raw, ev);
-    launch_z2<false>(K2, F.len[2].tw, real, cplx, (int)nrows, st);
+    launch_z2<false>(K2, F.len[2].tw, real, cplx, (int)nrows, ZeroWords{}, st);
     return 2;
   }
   if (zy == ZY_GROUPS) {
     launch_groups_y(Gy, false, zy_geom(F, cell), cplx, partials, nblocks, raw, ev, st);
-    launch_groups_z(Gz, false, real, cplx, plane ? K0 : 1, plane ? K1 : (int)nrows, st);
+    launch_groups_z(Gz, false, real, cplx, plane ? K0 : 1, plane ? K1 : (int)nrows, ZeroWords{}, st);
     return 2;
   }
   int k = 0;
@@ -1084,18 +1089,10 @@ static int x_pass(const FftPlan3 &F, const Geom &g, const Influence &inf, const 
 }
 
 int launch_fft_forward(const FftPlan3 &F, const Geom &g, const float *real, float2 *cplx, const DeconvArgs &dc,
-                       cudaStream_t st) {
+                       const ZeroWords &zw, cudaStream_t st) {
   int nb;
   Influence none{};
-  return fwd_zy(F, real, cplx, st) + x_pass<XM_FWD_DECONV>(F, g, none, dc.iB0, dc.iB1, dc.iB2, cplx, nullptr, nb, st);
-}
-
-int launch_conv_inverse(const FftPlan3 &F, const Geom &g, const Influence &inf, const double *iB0,
-                        const double *iB1, const double *iB2, float2 *cplx, float *real, double *partials,
-                        double *raw, double *ev, cudaStream_t st) {
-  int nb;
-  int k = x_pass<XM_CONV_INV>(F, g, inf, iB0, iB1, iB2, cplx, partials, nb, st);
-  return k + inv_yz(F, cplx, real, partials, nb, g.cell, raw, ev, st);
+  return fwd_zy(F, real, cplx, zw, st) + x_pass<XM_FWD_DECONV>(F, g, none, dc.iB0, dc.iB1, dc.iB2, cplx, nullptr, nb, st);
 }
 
 int launch_conv_energy(const FftPlan3 &F, const Geom &g, const Influence &inf, const double *iB0, const double *iB1,
@@ -1115,15 +1112,6 @@ int launch_energy(const FftPlan3 &F, const Geom &g, const Influence &inf, const 
 int launch_x_conv(const FftPlan3 &F, const Geom &g, const Influence &inf, const double *iB0, const double *iB1,
                   const double *iB2, float2 *cplx, double *partials, int &nblocks, cudaStream_t st) {
   return x_pass<XM_FWD_CONV_INV>(F, g, inf, iB0, iB1, iB2, cplx, partials, nblocks, st);
-}
-
-int launch_fft_conv_solve(const FftPlan3 &F, const Geom &g, const Influence &inf, const double *iB0,
-                          const double *iB1, const double *iB2, const float *real_in, float2 *cplx,
-                          float *real_out, double *partials, double *raw, double *ev, cudaStream_t st) {
-  int nb;
-  int k = fwd_zy(F, real_in, cplx, st);
-  k += x_pass<XM_FWD_CONV_INV>(F, g, inf, iB0, iB1, iB2, cplx, partials, nb, st);
-  return k + inv_yz(F, cplx, real_out, partials, nb, g.cell, raw, ev, st);
 }
 
 }  // namespace spme

@@ -129,7 +129,8 @@ constexpr int kGzWarps = 4;
 template <int G>
 __global__ void __launch_bounds__(32 * kGzWarps) fft_gz_r2c_kernel(FftGroups F, const float *__restrict__ rin,
                                                                    float2 *__restrict__ cout, int nlines, int rpp,
-                                                                   FastDiv lpp) {
+                                                                   FastDiv lpp, ZeroWords zw) {
+  zero_words(zw);
   extern __shared__ float2 sm[];
   constexpr int LW = 32 / G;
   const int n = F.n, n1 = F.n1, n2 = F.n2, ldim = n / 2 + 1, ep = n2 | 1;
@@ -446,7 +447,8 @@ void fft_groups_prepare() {
 }
 
 template <bool FWD>
-static void launch_gz(const FftGroups &F, float *real, float2 *cplx, int planes, int rpp, cudaStream_t st) {
+static void launch_gz(const FftGroups &F, float *real, float2 *cplx, int planes, int rpp, const ZeroWords &zw,
+                      cudaStream_t st) {
   const int m = F.n1 > F.n2 ? F.n1 : F.n2;
   const int G = m <= 8 ? 8 : (m <= 16 ? 16 : 32), lw = 32 / G;
   const int lines = planes * ((rpp + 1) / 2);
@@ -458,7 +460,7 @@ static void launch_gz(const FftGroups &F, float *real, float2 *cplx, int planes,
   const unsigned blocks = (unsigned)((warps + wpc - 1) / wpc);
   auto go = [&](auto GC) {
     constexpr int GG = decltype(GC)::value;
-    if (FWD) fft_gz_r2c_kernel<GG><<<blocks, 32 * wpc, smem, st>>>(F, real, cplx, lines, rpp, lpp);
+    if (FWD) fft_gz_r2c_kernel<GG><<<blocks, 32 * wpc, smem, st>>>(F, real, cplx, lines, rpp, lpp, zw);
     else fft_gz_c2r_kernel<GG><<<blocks, 32 * wpc, smem, st>>>(F, cplx, real, lines, rpp, lpp);
   };
   if (G == 8) go(std::integral_constant<int, 8>{});
@@ -466,9 +468,9 @@ static void launch_gz(const FftGroups &F, float *real, float2 *cplx, int planes,
   else go(std::integral_constant<int, 32>{});
 }
 void launch_groups_z(const FftGroups &F, bool forward, float *real, float2 *cplx, int planes, int rpp,
-                     cudaStream_t st) {
-  if (forward) launch_gz<true>(F, real, cplx, planes, rpp, st);
-  else launch_gz<false>(F, real, cplx, planes, rpp, st);
+                     const ZeroWords &zw, cudaStream_t st) {
+  if (forward) launch_gz<true>(F, real, cplx, planes, rpp, zw, st);
+  else launch_gz<false>(F, real, cplx, planes, rpp, zw, st);
 }
 
 // Lines per CTA (8 to 32): CTAs of at least 128 (y) or 256 (x) threads, at

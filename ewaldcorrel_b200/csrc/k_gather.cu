@@ -576,6 +576,8 @@ static bool use_tiles(const Geom &g, int n) {
   return g.order >= 6 && n >= ((g.K2 & 1) ? kTileMinPointsOdd : kTileMinPoints);
 }
 
+bool gather_uses_buckets(const Geom &g, int n, bool dx, bool phi) { return n > 0 && (dx || phi) && use_tiles(g, n); }
+
 void gather_prepare() {
   gather_tile_attr<6, kTileX, kTileY, kTileThreads>();
   gather_tile_attr<8, kTileX, kTileY, kTileThreads>();

@@ -249,7 +249,8 @@ long sort_buckets(const Geom &g, int zshift) {
   return (long)g.K0 * g.K1 * nzb;
 }
 
-// Word layout of the bucket-count region (zeroed before every sort):
+// Word layout of the bucket-count region (zero before every sort: by a memset,
+// or by a kernel that runs after the last use of the previous sort's):
 //   [0, nb + 1)            counts, then offsets
 //   [nb + 1, 2 nb + 1)     head: atoms of each bucket in its first H - 1 cells
 //   [2 nb + 1, 3 nb + 1)   tail: atoms of each bucket in its last H cells
@@ -760,8 +761,14 @@ void sort_prepare() {
 // On return (stream order): keys[0] / vals[0] hold the stable order,
 // rec_sorted the records in that order, cell_start the bucket offsets
 // (sort_buckets(g, zshift) + 1 of them).
+ZeroWords sort_count_words(const Geom &g, int n, const SortBuffers &b, int zshift) {
+  const long nb = sort_buckets(g, zshift);
+  return ZeroWords{reinterpret_cast<uint32_t *>(b.cell_start),
+                   (long)cell_count_words(nb, n < 0 ? b.slots != nullptr : use_slots(g, n, b, zshift))};
+}
+
 int launch_cell_sort(const Geom &g, int n, const double *x, const double *w, SortBuffers &b, cudaStream_t st,
-                     int zshift) {
+                     int zshift, bool clean) {
   const long nb = sort_buckets(g, zshift);
   const long ntiles = cell_tiles(nb);
   const int tshift = cell_tile_shift(nb);
@@ -780,7 +787,7 @@ int launch_cell_sort(const Geom &g, int n, const double *x, const double *w, Sor
   // tile sums taken while counting, while they are few (more: one pass over the counts)
   const bool count_tiles = ntiles > 1 && ntiles <= kCountTiles && n > 0;
   const Slots sl{slots ? b.slots : nullptr, b.nslot, spill, b.next, (uint32_t)nb};
-  cudaMemsetAsync(count, 0, sizeof(uint32_t) * (3 * nb + 1 + ntiles + (slots ? nb : 0)), st);
+  if (!clean) cudaMemsetAsync(count, 0, sizeof(uint32_t) * cell_count_words(nb, slots), st);
   int launches = 0;
   if (n > 0) {
     key_count_kernel<<<ceil_div(n, 256), 256, 0, st>>>(g, n, x, w, b.keys[1], b.vals[1], b.rec, count, bm,

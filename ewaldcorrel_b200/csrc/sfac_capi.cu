@@ -466,7 +466,9 @@ void *sfac_ctor(double L[6], int K[3], int order) {
       n += fft_make_len(h->fft.len[d], K[d], h->d_tw[d], h->stream);
       n += launch_bspline_moduli(K[d], order, h->nodes, h->d_iB[d], h->stream);
     }
-    ok = launched(h, n, "ctor kernels") && CK(h, cudaMemsetAsync(h->d_real, 0, sizeof(float) * h->nreal, h->stream)) &&
+    const ZeroWords counts = sort_count_words(g, -1, h->sb, kSpreadZShift);
+    ok = launched(h, n, "ctor kernels") && CK(h, cudaMemsetAsync(counts.p, 0, sizeof(uint32_t) * counts.n, h->stream)) &&
+         CK(h, cudaMemsetAsync(h->d_real, 0, sizeof(float) * h->nreal, h->stream)) &&
          CK(h, cudaMemsetAsync(h->d_cplx, 0, sizeof(float2) * h->nmodes, h->stream)) && sync(h);
   }
   if (!ok) {
@@ -494,11 +496,12 @@ void sfac(void *p, int n, const double *w, const double *x) {
       return;
   }
   CK(h, cudaEventRecord(h->ev_in, h->stream));
-  int k = launch_cell_sort(h->geom, n, h->d_x, h->d_w, h->sb, h->stream, kSpreadZShift);
+  int k = launch_cell_sort(h->geom, n, h->d_x, h->d_w, h->sb, h->stream, kSpreadZShift, true);
   k += launch_spread(h->geom, h->spline, h->sb.cell_start, h->sb.keys[h->sb.cur], h->sb.rec_sorted, h->d_real,
                      h->stream);
   DeconvArgs dc{h->d_iB[0], h->d_iB[1], h->d_iB[2], h->ldim};
-  k += launch_fft_forward(h->fft, h->geom, h->d_real, h->d_cplx, dc, h->stream);
+  k += launch_fft_forward(h->fft, h->geom, h->d_real, h->d_cplx, dc,
+                          sort_count_words(h->geom, n, h->sb, kSpreadZShift), h->stream);
   if (!launched(h, k, "sfac kernels")) return;
   // The caller may reuse w and x once this returns: wait for the copies only.
   CK(h, cudaEventSynchronize(h->ev_in));
@@ -1059,10 +1062,16 @@ static int enqueue_solve(Handle *h, int n, const double *x, const double *w, dou
                          double *ev, double *dEdL, bool timed) {
   cudaStream_t st = h->stream;
   int k = 0;
+  // The sort's count words are zero between calls: the first FFT pass after
+  // the spread zeroes them, or a memset at the end where the gather still
+  // reads the bucket offsets.  (A memset before the sort was one more
+  // dependent graph node at the head of every solve.)
+  const ZeroWords counts = sort_count_words(h->geom, n, h->sb, kSpreadZShift);
+  const bool late = !dEdL && gather_uses_buckets(h->geom, n, dx != nullptr, phi != nullptr);
   if (timed) CK(h, cudaEventRecord(h->ev_stage[0], st));
   {
     Nvtx r("spme cell sort");
-    k += launch_cell_sort(h->geom, n, x, w, h->sb, st, kSpreadZShift);
+    k += launch_cell_sort(h->geom, n, x, w, h->sb, st, kSpreadZShift, true);
   }
   if (timed) CK(h, cudaEventRecord(h->ev_stage[1], st));
   {
@@ -1073,7 +1082,7 @@ static int enqueue_solve(Handle *h, int n, const double *x, const double *w, dou
   int nb = 0;
   {
     Nvtx r("spme fft forward");
-    k += fwd_zy(h->fft, h->d_real, h->d_cplx, st);
+    k += fwd_zy(h->fft, h->d_real, h->d_cplx, late ? ZeroWords{} : counts, st);
   }
   if (timed) CK(h, cudaEventRecord(h->ev_stage[3], st));
   {
@@ -1096,6 +1105,7 @@ static int enqueue_solve(Handle *h, int n, const double *x, const double *w, dou
   else if (n > 0 && (dx || phi))
     k += launch_gather(h->geom, h->spline, n, x, w, h->d_real, dx, phi, st, perm, skeys, h->sb.rec_sorted,
                        h->sb.cell_start);
+  if (late) CK(h, cudaMemsetAsync(counts.p, 0, sizeof(uint32_t) * counts.n, st));
   if (timed) CK(h, cudaEventRecord(h->ev_stage[6], st));
   return k;
 }

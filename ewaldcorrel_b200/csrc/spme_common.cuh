@@ -97,6 +97,18 @@ struct FastDiv {
   }
 };
 
+// Words that a kernel sets to zero beside its own work (the cell sort's counts
+// for the next sort): n words at p, p 16-byte aligned.
+struct ZeroWords {
+  uint32_t *p;
+  long n;
+};
+__device__ __forceinline__ void zero_words(const ZeroWords &z) {
+  const long i0 = (long)blockIdx.x * blockDim.x + threadIdx.x, step = (long)gridDim.x * blockDim.x;
+  for (long i = i0; i < z.n / 4; i += step) reinterpret_cast<uint4 *>(z.p)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (i0 < (z.n & 3)) z.p[(z.n & ~3L) + i0] = 0u;
+}
+
 // M_n(t + j) by Horner (BSpline::bspl_coef, sfac.hpp:124-131), FP32.
 __device__ __forceinline__ float bspl_eval(const Spline &S, int n, float t, int j) {
   const float *r = S.c + j * n;

@@ -48,8 +48,12 @@ size_t cell_count_words(long nbuckets, bool with_slots);
 // the bucket's own 32 points take on the real grid, which is free until the
 // spread writes it and lends the space.
 constexpr int kSpreadSlots = 16;
+// clean: the count words are zero already (sort_count_words), no memset.
 int launch_cell_sort(const Geom &g, int n, const double *x, const double *w, SortBuffers &b, cudaStream_t st,
-                     int zshift);
+                     int zshift, bool clean);
+// The words of b that a sort of n atoms leaves to be zeroed (n < 0: all that
+// any sort wants zero on entry).
+ZeroWords sort_count_words(const Geom &g, int n, const SortBuffers &b, int zshift);
 void sort_prepare();  // sets the one-CTA sort's shared-memory limit once (before any graph capture)
 
 // ---- spread (k_spread.cu) ----
@@ -90,36 +94,28 @@ bool fft_plane_fits(int K1, int K2);
 long fft_x_blocks_max(int K1, int K2);  // upper bound of x-pass CTAs (energy/virial partials)
 // sfac path: forward 3D r2c and division by the moduli -> S.
 int launch_fft_forward(const FftPlan3 &F, const Geom &g, const float *real, float2 *cplx, const DeconvArgs &dc,
-                       cudaStream_t st);
-// de1 path: S -> energy/virial (ev, raw sums) and the real potential grid.
-int launch_conv_inverse(const FftPlan3 &F, const Geom &g, const Influence &inf, const double *iB0,
-                        const double *iB1, const double *iB2, float2 *cplx, float *real, double *partials,
-                        double *raw, double *ev, cudaStream_t st);
+                       const ZeroWords &zw, cudaStream_t st);
 // de1's first half: x pass with the convolution, and the energy/virial sums
-// in raw (the same sums, in the same order, as launch_conv_inverse forms);
+// in raw (the same sums, in the same order, as en forms);
 // the caller enqueues inv_yz (without partials) afterwards.
 int launch_conv_energy(const FftPlan3 &F, const Geom &g, const Influence &inf, const double *iB0, const double *iB1,
                        const double *iB2, float2 *cplx, double *partials, double *raw, cudaStream_t st);
-// en path: energy/virial sums of S (raw), same order as launch_conv_inverse.
+// en path: energy/virial sums of S (raw), same order as launch_conv_energy.
 int launch_energy(const FftPlan3 &F, const Geom &g, const Influence &inf, const double *iB0, const double *iB1,
                   const double *iB2, float2 *cplx, double *partials, double *raw, cudaStream_t st);
 // The three launches of the fused solve, also callable one by one:
 // forward z/y; x forward + convolution + x inverse; inverse y/z (+ reduction).
-int fwd_zy(const FftPlan3 &F, const float *real, float2 *cplx, cudaStream_t st);
+int fwd_zy(const FftPlan3 &F, const float *real, float2 *cplx, const ZeroWords &zw, cudaStream_t st);
 int launch_x_conv(const FftPlan3 &F, const Geom &g, const Influence &inf, const double *iB0, const double *iB1,
                   const double *iB2, float2 *cplx, double *partials, int &nblocks, cudaStream_t st);
 int inv_yz(const FftPlan3 &F, float2 *cplx, float *real, const double *partials, int nblocks,
            const CellConst *cell, double *raw, double *ev, cudaStream_t st);
-// fused solve: spread grid -> energy/virial and potential grid.
-int launch_fft_conv_solve(const FftPlan3 &F, const Geom &g, const Influence &inf, const double *iB0,
-                          const double *iB1, const double *iB2, const float *real_in, float2 *cplx,
-                          float *real_out, double *partials, double *raw, double *ev, cudaStream_t st);
-
 // ---- FFT passes by groups of stages (k_fft_groups.cu) ----
 bool fft_group_split(const FftLen &L, FftGroups &G);
 void fft_groups_prepare();  // sets shared-memory limits once (before any graph capture)
 // planes x rpp rows, paired within each plane
-void launch_groups_z(const FftGroups &F, bool forward, float *real, float2 *cplx, int planes, int rpp, cudaStream_t st);
+void launch_groups_z(const FftGroups &F, bool forward, float *real, float2 *cplx, int planes, int rpp,
+                     const ZeroWords &zw, cudaStream_t st);
 void launch_groups_y(const FftGroups &F, bool forward, const Geom &g, float2 *cplx, const double *partials, int nblocks,
                      double *raw, double *ev, cudaStream_t st);
 void launch_groups_x(const FftGroups &F, int mode, const Geom &g, const Influence &inf, const double *iB0,
@@ -196,6 +192,7 @@ int launch_finish(const double *partials, int nblocks, const CellConst *cell, do
 int launch_gather(const Geom &g, const Spline &S, int n, const double *x, const double *w,
                   const float *grid, double *dx, double *phi, cudaStream_t st, const uint32_t *perm = nullptr,
                   const uint32_t *keys = nullptr, const float4 *rec = nullptr, const int *cs = nullptr);
+bool gather_uses_buckets(const Geom &g, int n, bool dx, bool phi);  // whether a launch_gather given cs reads it
 void gather_prepare();  // sets the brick kernels' shared-memory limits once (before any graph capture)
 // Gather + cell adjoint: dE/dL (6 doubles, device) from dE/dx, the virial in ev
 // and the positions; cellp is scratch of gather_cell_words(n) doubles.
