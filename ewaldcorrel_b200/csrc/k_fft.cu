@@ -845,13 +845,15 @@ bool fft_plane_fits(int K1, int K2) {
 long fft_x_blocks_max(int K1, int K2) { return ((long)K1 * (K2 / 2 + 1) + 7) / 8; }
 
 // Shape of a two-level per-axis pass over `nlines` lines of length n:
-// B = 2^lgB lines per CTA (8..32), B*max(n1, n2) threads (at most 512), B halved while fewer than two CTAs per SM
+// B = 2^lgB lines per CTA (8..32; at least 256 threads: 16 lines, 128-byte
+// pieces of memory, at 256^3, where the solve took 655.3 us against 660.3 with
+// 8), B*max(n1, n2) threads (at most 512), B halved while fewer than two CTAs per SM
 // (148 SMs) would run.  False when n has no n1 * n2 split.
 static bool lines2_shape(int n, long nlines, int &n1, int &n2, int &lgB, int &threads) {
   if (!rdft::split_line(n, n1, n2)) return false;
   const int m = n1 > n2 ? n1 : n2;
   int B = 8;
-  while (B < 32 && B * m < 128) B <<= 1;
+  while (B < 32 && B * m < 256) B <<= 1;
   while (B > 8 && (nlines + B - 1) / B < 2 * 148) B >>= 1;
   while (B > 8 && B * m > 512) B >>= 1;
   if (B * m > 512) return false;

@@ -31,44 +31,32 @@ __device__ __forceinline__ void wrap_run(int o, int K, int (&idx)[P]) {
   }
 }
 
-// Order-P stencil sum of the grid around one point, factorised per axis:
-// pot = sum_i wx_i sum_j wy_j sum_k wz_k Q, and the three derivatives.
-// WRAP false: the z indices are z0 .. z0 + P - 1; true: iz[k] (z0 = 0).
+// Sums of one x plane of the stencil, sy = sum_j wy_j sum_k wz_k Q and the two
+// with a derivative: pl points at the plane's first value of the run in z.
+// WRAP false: the z indices are 0 .. P - 1; true: iz[k].
 template <int P, bool WRAP>
-__device__ __forceinline__ void stencil_sum(const float *__restrict__ grid, const Geom &g, int o0,
-                                            const int (&iy)[P], int z0, const int (&iz)[P], const float (&wx)[P],
-                                            const float (&dwx)[P], const float (&wy)[P], const float (&dwy)[P],
-                                            const float (&wz)[P], const float (&dwz)[P], float &pot, float &gx,
-                                            float &gy, float &gz) {
-  const long plane = (long)g.K1 * g.K2;
-  int xi = o0;  // (o0 + i) mod K0
-#pragma unroll 1
-  for (int i = 0; i < P; i++, xi = (xi + 1 == g.K0) ? 0 : xi + 1) {
-    const float *pl = grid + xi * plane + z0;
-    float sy = 0.f, dy = 0.f, dz = 0.f;
+__device__ __forceinline__ void plane_sum(const float *__restrict__ grid, const Geom &g, const float *pl,
+                                          const int (&iy)[P], const int (&iz)[P], const float (&wy)[P],
+                                          const float (&dwy)[P], const float (&wz)[P], const float (&dwz)[P], float &sy,
+                                          float &dy, float &dz) {
+  sy = dy = dz = 0.f;
 #pragma unroll
-    for (int j = 0; j < P; j++) {
-      const float *col = pl + (long)iy[j] * g.K2;
-      float sz = 0.f, dzz = 0.f;
+  for (int j = 0; j < P; j++) {
+    const float *col = pl + (long)iy[j] * g.K2;
+    float sz = 0.f, dzz = 0.f;
 #pragma unroll
-      for (int k = 0; k < P; k++) {
-        const float q = SPME_IN(col + (WRAP ? iz[k] : k) - grid, g.K0 * plane, CK_GATHER_GRID)
-                            ? __ldg(col + (WRAP ? iz[k] : k))
-                            : 0.f;
-        sz = fmaf(wz[k], q, sz);
-        dzz = fmaf(dwz[k], q, dzz);
-      }
-      sy = fmaf(wy[j], sz, sy);
-      dy = fmaf(dwy[j], sz, dy);
-      dz = fmaf(wy[j], dzz, dz);
+    for (int k = 0; k < P; k++) {
+      const float q = SPME_IN(col + (WRAP ? iz[k] : k) - grid, (long)g.K0 * g.K1 * g.K2, CK_GATHER_GRID)
+                          ? __ldg(col + (WRAP ? iz[k] : k))
+                          : 0.f;
+      sz = fmaf(wz[k], q, sz);
+      dzz = fmaf(dwz[k], q, dzz);
     }
-    pot = fmaf(wx[i], sy, pot);
-    gx = fmaf(dwx[i], sy, gx);
-    gy = fmaf(wx[i], dy, gy);
-    gz = fmaf(wx[i], dz, gz);
+    sy = fmaf(wy[j], sz, sy);
+    dy = fmaf(dwy[j], sz, dy);
+    dz = fmaf(wy[j], dzz, dz);
   }
 }
-
 
 // Vector width of the row loads: each z run of P values is read as W / kVW
 // aligned float2 loads from zb = o2 rounded down to even (W = P + 2 values,
@@ -79,41 +67,88 @@ __device__ __forceinline__ void stencil_sum(const float *__restrict__ grid, cons
 constexpr int kVW = 2;  // float2
 template <int P> struct VecWin { static constexpr int W = (P + kVW - 1 + kVW - 1) / kVW * kVW; };
 
-// Row sums from aligned vector loads: the window [zb, zb + W) holds the run,
-// the weights are pre-shifted (zeros outside the run).
+// The same from aligned vector loads: the window of W values at pl holds the
+// run, the weights are pre-shifted (zeros outside the run).
 template <int P>
-__device__ __forceinline__ void stencil_sum_vec(const float *__restrict__ grid, const Geom &g, int o0,
-                                                const int (&iy)[P], int zb, const float (&wz)[VecWin<P>::W],
-                                                const float (&dwz)[VecWin<P>::W], const float (&wx)[P],
-                                                const float (&dwx)[P], const float (&wy)[P], const float (&dwy)[P],
-                                                float &pot, float &gx, float &gy, float &gz) {
-  constexpr int W = VecWin<P>::W;
-  const long plane = (long)g.K1 * g.K2;
-  int xi = o0;
+__device__ __forceinline__ void plane_sum_vec(const float *__restrict__ grid, const Geom &g, const float *pl,
+                                              const int (&iy)[P], const float (&wy)[P], const float (&dwy)[P],
+                                              const float (&wz)[VecWin<P>::W], const float (&dwz)[VecWin<P>::W],
+                                              float &sy, float &dy, float &dz) {
+  sy = dy = dz = 0.f;
+#pragma unroll
+  for (int j = 0; j < P; j++) {
+    const float *col = pl + (long)iy[j] * g.K2;
+    float sz = 0.f, dzz = 0.f;
+#pragma unroll
+    for (int v = 0; v < VecWin<P>::W / kVW; v++) {
+      const float2 q = SPME_IN(col + 2 * v + 1 - grid, (long)g.K0 * g.K1 * g.K2, CK_GATHER_GRID)
+                           ? __ldg(reinterpret_cast<const float2 *>(col) + v)
+                           : make_float2(0.f, 0.f);
+      sz = fmaf(wz[2 * v], q.x, sz); dzz = fmaf(dwz[2 * v], q.x, dzz);
+      sz = fmaf(wz[2 * v + 1], q.y, sz); dzz = fmaf(dwz[2 * v + 1], q.y, dzz);
+    }
+    sy = fmaf(wy[j], sz, sy);
+    dy = fmaf(dwy[j], sz, dy);
+    dz = fmaf(wy[j], dzz, dz);
+  }
+}
+
+// Order-P stencil sum of the grid around one point, factorised per axis:
+// pot = sum_i wx_i sum_j wy_j sum_k wz_k Q, and the three derivatives, the
+// planes in order.  plane(xi, sy, dy, dz): the sums of grid plane xi.
+template <int P, class F>
+__device__ __forceinline__ void stencil_sum(const Geom &g, int o0, const float (&wx)[P], const float (&dwx)[P],
+                                            F &&plane, float &pot, float &gx, float &gy, float &gz) {
+  int xi = o0;  // (o0 + i) mod K0
 #pragma unroll 1
   for (int i = 0; i < P; i++, xi = (xi + 1 == g.K0) ? 0 : xi + 1) {
-    const float *pl = grid + xi * plane + zb;
-    float sy = 0.f, dy = 0.f, dz = 0.f;
-#pragma unroll
-    for (int j = 0; j < P; j++) {
-      const float *col = pl + (long)iy[j] * g.K2;
-      float sz = 0.f, dzz = 0.f;
-#pragma unroll
-      for (int v = 0; v < W / kVW; v++) {
-        const float2 q = SPME_IN(col + 2 * v + 1 - grid, g.K0 * plane, CK_GATHER_GRID)
-                             ? __ldg(reinterpret_cast<const float2 *>(col) + v)
-                             : make_float2(0.f, 0.f);
-        sz = fmaf(wz[2 * v], q.x, sz); dzz = fmaf(dwz[2 * v], q.x, dzz);
-        sz = fmaf(wz[2 * v + 1], q.y, sz); dzz = fmaf(dwz[2 * v + 1], q.y, dzz);
-      }
-      sy = fmaf(wy[j], sz, sy);
-      dy = fmaf(dwy[j], sz, dy);
-      dz = fmaf(wy[j], dzz, dz);
-    }
+    float sy, dy, dz;
+    plane(xi, sy, dy, dz);
     pot = fmaf(wx[i], sy, pot);
     gx = fmaf(dwx[i], sy, gx);
     gy = fmaf(wx[i], dy, gy);
     gz = fmaf(wx[i], dz, gz);
+  }
+}
+
+// Calls f with the plane sums of a point whose z run starts at o2, as a
+// function of the plane: f([](xi, sy, dy, dz)).  The choice between vector
+// loads, plain loads and wrapped indices is warp-uniform (no divergent second
+// copy of the stencil); it depends on nothing but the active lanes' o2.
+template <int P, class F>
+__device__ __forceinline__ void with_planes(const float *__restrict__ grid, const Geom &g, const int (&iy)[P], int o2,
+                                            const float (&wy)[P], const float (&dwy)[P], const float (&wz)[P],
+                                            const float (&dwz)[P], F &&f) {
+  const long plane = (long)g.K1 * g.K2;
+  int iz[P];
+  const int sh = o2 & (kVW - 1), zb = o2 - sh;
+  if ((g.K2 % kVW) == 0 && __all_sync(__activemask(), zb + VecWin<P>::W <= g.K2)) {
+    constexpr int W = VecWin<P>::W;
+    float wzv[W], dwzv[W];
+#pragma unroll
+    for (int k = 0; k < W; k++) {
+      float v = 0.f, d = 0.f;
+#pragma unroll
+      for (int t = 0; t < kVW; t++)
+        if (k - t >= 0 && k - t < P) {
+          v = (sh == t) ? wz[k - t] : v;
+          d = (sh == t) ? dwz[k - t] : d;
+        }
+      wzv[k] = v;
+      dwzv[k] = d;
+    }
+    f([&](int xi, float &sy, float &dy, float &dz) {
+      plane_sum_vec<P>(grid, g, grid + xi * plane + zb, iy, wy, dwy, wzv, dwzv, sy, dy, dz);
+    });
+  } else if (__all_sync(__activemask(), o2 + P <= g.K2)) {
+    f([&](int xi, float &sy, float &dy, float &dz) {
+      plane_sum<P, false>(grid, g, grid + xi * plane + o2, iy, iz, wy, dwy, wz, dwz, sy, dy, dz);
+    });
+  } else {
+    wrap_run<P>(o2, g.K2, iz);
+    f([&](int xi, float &sy, float &dy, float &dz) {
+      plane_sum<P, true>(grid, g, grid + xi * plane, iy, iz, wy, dwy, wz, dwz, sy, dy, dz);
+    });
   }
 }
 
@@ -125,6 +160,48 @@ struct SortedView {
   const float4 *rec;
   FastDiv K2d, K12d;  // division by K2 and by K1*K2
 };
+
+// A point's input index, stencil origin (wrapped) and B-spline arguments; see
+// gather_kernel for SORTED.
+struct PointAt {
+  int a, o0, o1, o2;
+  float t0, t1, t2;
+};
+template <int P, bool SORTED>
+__device__ __forceinline__ PointAt point_at(const Geom &g, int r, int n, const double *__restrict__ x,
+                                            const SortedView &sv) {
+  PointAt p;
+  if (SORTED) {
+    p.a = (int)sv.perm[r];
+    uint32_t key = sv.key[r];
+    // a failed check substitutes atom 0 / key 0 (the run is flagged already)
+    if (!SPME_IN(p.a, n, CK_GATHER_ATOM)) p.a = 0;
+    if (!SPME_IN(key, (long)g.K0 * g.K1 * g.K2, CK_GATHER_KEY)) key = 0;
+    const float4 u = sv.rec[r];
+    const uint32_t n0 = sv.K12d.div(key), rem = key - n0 * (uint32_t)(g.K1 * g.K2);
+    const uint32_t n1 = sv.K2d.div(rem), n2 = rem - n1 * (uint32_t)g.K2;
+    p.o0 = imod((int)n0 + 1 - P / 2, g.K0);
+    p.o1 = imod((int)n1 + 1 - P / 2, g.K1);
+    p.o2 = imod((int)n2 + 1 - P / 2, g.K2);
+    p.t0 = 1.f - u.x;
+    p.t1 = 1.f - u.y;
+    p.t2 = 1.f - u.z;
+  } else {
+    const CellConst cc = *g.cell;
+    p.a = r;
+    double s0, s1, s2;
+    frac_coords(cc, x[3 * r + 0], x[3 * r + 1], x[3 * r + 2], s0, s1, s2);
+    const double u0 = __dmul_rn(s0, (double)g.K0), u1 = __dmul_rn(s1, (double)g.K1), u2 = __dmul_rn(s2, (double)g.K2);
+    const int c0 = (int)ceil(u0), c1 = (int)ceil(u1), c2 = (int)ceil(u2);
+    p.t0 = (float)((double)c0 - u0);
+    p.t1 = (float)((double)c1 - u1);
+    p.t2 = (float)((double)c2 - u2);
+    p.o0 = imod(c0 - P / 2, g.K0);
+    p.o1 = imod(c1 - P / 2, g.K1);
+    p.o2 = imod(c2 - P / 2, g.K2);
+  }
+  return p;
+}
 
 // CELL: also the per-block sums of s_i (dE/dr)_j over the block's points
 // (s = iL^T x, unwrapped), written to cellp[block][9] in a fixed order.
@@ -146,37 +223,9 @@ __global__ void __launch_bounds__(256, CELL ? 2 : 3) gather_kernel(Geom g, Splin
   }
   if (r < n) {
     const CellConst cc = *g.cell;
-    int a, o0, o1, o2;
-    float t0, t1, t2;
-    if (SORTED) {
-      a = (int)sv.perm[r];
-      uint32_t key = sv.key[r];
-      // a failed check substitutes atom 0 / key 0 (the run is flagged already)
-      if (!SPME_IN(a, n, CK_GATHER_ATOM)) a = 0;
-      if (!SPME_IN(key, (long)g.K0 * g.K1 * g.K2, CK_GATHER_KEY)) key = 0;
-      const float4 u = sv.rec[r];
-      const uint32_t n0 = sv.K12d.div(key), rem = key - n0 * (uint32_t)(g.K1 * g.K2);
-      const uint32_t n1 = sv.K2d.div(rem), n2 = rem - n1 * (uint32_t)g.K2;
-      o0 = imod((int)n0 + 1 - P / 2, g.K0);
-      o1 = imod((int)n1 + 1 - P / 2, g.K1);
-      o2 = imod((int)n2 + 1 - P / 2, g.K2);
-      t0 = 1.f - u.x;
-      t1 = 1.f - u.y;
-      t2 = 1.f - u.z;
-    } else {
-      a = r;
-      double s0, s1, s2;
-      frac_coords(cc, x[3 * a + 0], x[3 * a + 1], x[3 * a + 2], s0, s1, s2);
-      const double u0 = __dmul_rn(s0, (double)g.K0), u1 = __dmul_rn(s1, (double)g.K1),
-                   u2 = __dmul_rn(s2, (double)g.K2);
-      const int c0 = (int)ceil(u0), c1 = (int)ceil(u1), c2 = (int)ceil(u2);
-      t0 = (float)((double)c0 - u0);
-      t1 = (float)((double)c1 - u1);
-      t2 = (float)((double)c2 - u2);
-      o0 = imod(c0 - P / 2, g.K0);
-      o1 = imod(c1 - P / 2, g.K1);
-      o2 = imod(c2 - P / 2, g.K2);
-    }
+    const PointAt pt = point_at<P, SORTED>(g, r, n, x, sv);
+    const int a = pt.a, o0 = pt.o0, o1 = pt.o1, o2 = pt.o2;
+    const float t0 = pt.t0, t1 = pt.t1, t2 = pt.t2;
     float wx[P], dwx[P], wy[P], dwy[P], wz[P], dwz[P];
 #pragma unroll
     for (int i = 0; i < P; i++) {
@@ -187,32 +236,9 @@ __global__ void __launch_bounds__(256, CELL ? 2 : 3) gather_kernel(Geom g, Splin
     int iy[P];
     wrap_run<P>(o1, g.K1, iy);
     float pot = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
-    int iz[P];
-    // Warp-uniform choice (no divergent second copy of the stencil): when no
-    // active lane's z run wraps, constant offsets from one address per row.
-    const int sh = o2 & (kVW - 1), zb = o2 - sh;
-    if ((g.K2 % kVW) == 0 && __all_sync(__activemask(), zb + VecWin<P>::W <= g.K2)) {
-      constexpr int W = VecWin<P>::W;
-      float wzv[W], dwzv[W];
-#pragma unroll
-      for (int k = 0; k < W; k++) {
-        float v = 0.f, d = 0.f;
-#pragma unroll
-        for (int t = 0; t < kVW; t++)
-          if (k - t >= 0 && k - t < P) {
-            v = (sh == t) ? wz[k - t] : v;
-            d = (sh == t) ? dwz[k - t] : d;
-          }
-        wzv[k] = v;
-        dwzv[k] = d;
-      }
-      stencil_sum_vec<P>(grid, g, o0, iy, zb, wzv, dwzv, wx, dwx, wy, dwy, pot, gx, gy, gz);
-    } else if (__all_sync(__activemask(), o2 + P <= g.K2)) {
-      stencil_sum<P, false>(grid, g, o0, iy, o2, iz, wx, dwx, wy, dwy, wz, dwz, pot, gx, gy, gz);
-    } else {
-      wrap_run<P>(o2, g.K2, iz);
-      stencil_sum<P, true>(grid, g, o0, iy, 0, iz, wx, dwx, wy, dwy, wz, dwz, pot, gx, gy, gz);
-    }
+    with_planes<P>(grid, g, iy, o2, wy, dwy, wz, dwz, [&](auto &&plane) {
+      stencil_sum<P>(g, o0, wx, dwx, plane, pot, gx, gy, gz);
+    });
     if (GRAD) {
       const double f = -w[a] * cc.iV;
       const double G0 = (double)gx * f * g.K0, G1 = (double)gy * f * g.K1, G2 = (double)gz * f * g.K2;
@@ -266,6 +292,61 @@ __global__ void cell_grad_kernel(Geom g, const double *__restrict__ cellp, int n
   dEdL[3] = D[1][0];
   dEdL[4] = D[2][0];
   dEdL[5] = D[2][1];
+}
+
+// The same for few points: 8 lanes per point, lane i < P sums plane i, and the
+// point's first lane adds the planes in order (the same sums, so the same
+// bits).  With few points the thread-per-point kernel is one thread's chain of
+// P^2 row loads long while most of the chip idles.
+template <int P, bool GRAD, bool POT, bool SORTED>
+__global__ void __launch_bounds__(128) gather_split_kernel(Geom g, Spline S, int n, const double *__restrict__ x,
+                                                           const double *__restrict__ w,
+                                                           const float *__restrict__ grid, double *__restrict__ dx,
+                                                           double *__restrict__ phi, SortedView sv) {
+  const int r = blockIdx.x * (blockDim.x / 8) + threadIdx.x / 8, i = threadIdx.x & 7;
+  const bool live = r < n;
+  const PointAt pt = point_at<P, SORTED>(g, live ? r : n - 1, n, x, sv);
+  const int a = pt.a, o2 = pt.o2;
+  int xi = pt.o0 + min(i, P - 1);
+  if (xi >= g.K0) xi %= g.K0;
+  float wx = 0.f, dwx = 0.f, wy[P], dwy[P], wz[P], dwz[P];
+#pragma unroll
+  for (int k = 0; k < P; k++) {
+    float b, d;
+    dbspl_eval(S, P, pt.t0, k, b, d);
+    if (k == i) {
+      wx = b;
+      dwx = d;
+    }
+    dbspl_eval(S, P, pt.t1, k, wy[k], dwy[k]);
+    dbspl_eval(S, P, pt.t2, k, wz[k], dwz[k]);
+  }
+  int iy[P];
+  wrap_run<P>(pt.o1, g.K1, iy);
+  float sy = 0.f, dy = 0.f, dz = 0.f;
+  if (i < P)
+    with_planes<P>(grid, g, iy, o2, wy, dwy, wz, dwz, [&](auto &&plane) { plane(xi, sy, dy, dz); });
+  __syncwarp();
+  float pot = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
+#pragma unroll
+  for (int k = 0; k < P; k++) {  // every lane of the point adds the planes in order
+    const float wk = __shfl_sync(0xffffffffu, wx, k, 8), sk = __shfl_sync(0xffffffffu, sy, k, 8);
+    if (POT) pot = fmaf(wk, sk, pot);
+    if (GRAD) {
+      gx = fmaf(__shfl_sync(0xffffffffu, dwx, k, 8), sk, gx);
+      gy = fmaf(wk, __shfl_sync(0xffffffffu, dy, k, 8), gy);
+      gz = fmaf(wk, __shfl_sync(0xffffffffu, dz, k, 8), gz);
+    }
+  }
+  if (!live) return;
+  const CellConst cc = *g.cell;
+  if (GRAD && i < 3) {  // lane i writes component i
+    const double f = -w[a] * cc.iV;
+    const double G0 = (double)gx * f * g.K0, G1 = (double)gy * f * g.K1, G2 = (double)gz * f * g.K2;
+    dx[3 * a + i] = i == 0 ? cc.iL00 * G0
+                           : (i == 1 ? cc.iL10 * G0 + cc.iL11 * G1 : cc.iL20 * G0 + cc.iL21 * G1 + cc.iL22 * G2);
+  }
+  if (POT && i == 3) phi[a] = (double)pot * cc.iV;
 }
 
 // ---------------------------------------------------------------------------
@@ -589,6 +670,13 @@ void gather_prepare() {
 // but 4000 points at order 6 55.4 -> 57.5).
 constexpr int kGatherThreads = 128;
 
+// Points below which 8 lanes share one (orders 6 and 8).  Solves, thread per
+// point / 8 lanes, us: order 6, 500 points 43.1 / 35.0, 4000 55.4 / 49.0, 16k
+// 63.6 / 55.6, 32k 73.8 / 68.5, 50k 73.8 / 73.8; order 8, 4000 61.6 / 55.4, 16k
+// 69.7 / 65.7, 32k 84.1 / 84.0, 50k 90.2 / 92.4; order 4, 4000 43.1 / 43.1, 16k
+// 45.2 / 46.0 (not taken).
+constexpr int kSplitMaxPoints = 24576;
+
 template <int P, bool SORTED>
 static int gather_p(const Geom &g, const Spline &S, int n, const double *x, const double *w, const float *grid,
                     double *dx, double *phi, double *cellp, const SortedView &sv, cudaStream_t st) {
@@ -596,6 +684,18 @@ static int gather_p(const Geom &g, const Spline &S, int n, const double *x, cons
     gather_kernel<P, true, true, true, SORTED>
         <<<(n + 255) / 256, 256, 0, st>>>(g, S, n, x, w, grid, dx, phi, cellp, sv);
     return 1;
+  }
+  if constexpr (P >= 6) {
+    if (n <= kSplitMaxPoints && (dx || phi)) {
+      const int blocks = (n + 15) / 16;
+      if (dx && phi)
+        gather_split_kernel<P, true, true, SORTED><<<blocks, 128, 0, st>>>(g, S, n, x, w, grid, dx, phi, sv);
+      else if (dx)
+        gather_split_kernel<P, true, false, SORTED><<<blocks, 128, 0, st>>>(g, S, n, x, w, grid, dx, phi, sv);
+      else
+        gather_split_kernel<P, false, true, SORTED><<<blocks, 128, 0, st>>>(g, S, n, x, w, grid, dx, phi, sv);
+      return 1;
+    }
   }
   constexpr int threads = kGatherThreads;
   const int blocks = (n + threads - 1) / threads;
