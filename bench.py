@@ -194,12 +194,12 @@ NCU_TRAFFIC = {
 # Kernels of each stage (the roofline is reported for the longest stage that
 # is a single kernel launch).
 STAGE_KERNELS = {
-    "cell_sort": "key_count + tile_sum + cell_offsets + cell_scatter + cell_fixup (+ memset)",
+    "cell_sort": "key_count + cell_offsets + cell_place, or cell_scatter + cell_fixup",
     "spread": "spread_kernel",
-    "fft_forward": "fft_zr2c2_kernel + fft_y2_kernel<-1>",
+    "fft_forward": "fft_z2_r2c_kernel + fft_y2_kernel<-1>",
     "convolution": "fft_x2_kernel<XM_FWD_CONV_INV> (x FFT, Ewald convolution, energy/virial, inverse x FFT)",
-    "fft_inverse": "fft_y2_kernel<+1> (+ energy/virial reduction) + fft_zc2r2_kernel",
-    "gather": "gather_kernel (forces + potentials)",
+    "fft_inverse": "fft_y2_kernel<+1> (+ energy/virial reduction) + fft_z2_c2r_kernel",
+    "gather": "gather_tile_kernel or gather_kernel (forces + potentials)",
 }
 SINGLE_KERNEL_STAGES = ("spread", "convolution", "gather")
 

@@ -298,14 +298,13 @@ __global__ void cell_grad_kernel(Geom g, const double *__restrict__ cellp, int n
 // point's first lane adds the planes in order (the same sums, so the same
 // bits).  With few points the thread-per-point kernel is one thread's chain of
 // P^2 row loads long while most of the chip idles.
-template <int P, bool GRAD, bool POT, bool SORTED>
-__global__ void __launch_bounds__(128) gather_split_kernel(Geom g, Spline S, int n, const double *__restrict__ x,
-                                                           const double *__restrict__ w,
+template <int P, bool GRAD, bool POT>
+__global__ void __launch_bounds__(128) gather_split_kernel(Geom g, Spline S, int n, const double *__restrict__ w,
                                                            const float *__restrict__ grid, double *__restrict__ dx,
                                                            double *__restrict__ phi, SortedView sv) {
   const int r = blockIdx.x * (blockDim.x / 8) + threadIdx.x / 8, i = threadIdx.x & 7;
   const bool live = r < n;
-  const PointAt pt = point_at<P, SORTED>(g, live ? r : n - 1, n, x, sv);
+  const PointAt pt = point_at<P, true>(g, live ? r : n - 1, n, nullptr, sv);
   const int a = pt.a, o2 = pt.o2;
   int xi = pt.o0 + min(i, P - 1);
   if (xi >= g.K0) xi %= g.K0;
@@ -674,7 +673,8 @@ constexpr int kGatherThreads = 128;
 // point / 8 lanes, us: order 6, 500 points 43.1 / 35.0, 4000 55.4 / 49.0, 16k
 // 63.6 / 55.6, 32k 73.8 / 68.5, 50k 73.8 / 73.8; order 8, 4000 61.6 / 55.4, 16k
 // 69.7 / 65.7, 32k 84.1 / 84.0, 50k 90.2 / 92.4; order 4, 4000 43.1 / 43.1, 16k
-// 45.2 / 46.0 (not taken).
+// 45.2 / 46.0 (not taken).  Sorted points only: de2 of 24k points in input order
+// took 134 us with 8 lanes against 127, its lanes computing the FP64 origin 8 times.
 constexpr int kSplitMaxPoints = 24576;
 
 template <int P, bool SORTED>
@@ -685,15 +685,15 @@ static int gather_p(const Geom &g, const Spline &S, int n, const double *x, cons
         <<<(n + 255) / 256, 256, 0, st>>>(g, S, n, x, w, grid, dx, phi, cellp, sv);
     return 1;
   }
-  if constexpr (P >= 6) {
+  if constexpr (P >= 6 && SORTED) {
     if (n <= kSplitMaxPoints && (dx || phi)) {
       const int blocks = (n + 15) / 16;
       if (dx && phi)
-        gather_split_kernel<P, true, true, SORTED><<<blocks, 128, 0, st>>>(g, S, n, x, w, grid, dx, phi, sv);
+        gather_split_kernel<P, true, true><<<blocks, 128, 0, st>>>(g, S, n, w, grid, dx, phi, sv);
       else if (dx)
-        gather_split_kernel<P, true, false, SORTED><<<blocks, 128, 0, st>>>(g, S, n, x, w, grid, dx, phi, sv);
+        gather_split_kernel<P, true, false><<<blocks, 128, 0, st>>>(g, S, n, w, grid, dx, phi, sv);
       else
-        gather_split_kernel<P, false, true, SORTED><<<blocks, 128, 0, st>>>(g, S, n, x, w, grid, dx, phi, sv);
+        gather_split_kernel<P, false, true><<<blocks, 128, 0, st>>>(g, S, n, w, grid, dx, phi, sv);
       return 1;
     }
   }
