@@ -297,8 +297,12 @@ struct Slots {
 };
 
 // head/tail (may be null): see the word layout above; ht_h = H.  tsum (may be
-// null): the counts' tile sums, taken with one atomic per tile and CTA.
-constexpr int kCountTiles = 128;
+// null): the counts' tile sums, taken with one atomic per tile and CTA while
+// the tiles are few.  Solves with this / with tile_sum_kernel, us: 98k atoms on
+// 96^3 (4 tiles) 67.7 / 69.8, 200k on 128^3 (9) 123.2 / 125.6, 500k on 180^3 (24)
+// 289 / 286, 1M on 256^3 (65) 536.5 / 518: there every CTA's atoms meet every
+// tile, and a few thousand atomics on each sum take longer than the kernel.
+constexpr int kCountTiles = 16;
 __global__ void __launch_bounds__(256) key_count_kernel(Geom g, int n, const double *__restrict__ x,
                                                         const double *__restrict__ w, uint32_t *__restrict__ keys,
                                                         uint32_t *__restrict__ slot, float4 *__restrict__ rec,
