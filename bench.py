@@ -178,18 +178,16 @@ def algorithmic_bytes(n, K):
 
 # DRAM bytes (read + write) per launch of each stage's kernels, from ncu
 # captures of a plain solve (cold caches; summaries in profiles/).  Writes
-# that stay in the 126 MB L2 past the kernel's end are not counted.  At 256^3
-# the sort's figure is from profiles/dram_sort_triclinic1m.md, the spread's
-# from profiles/ncu_full_spread_triclinic1m.md, the x pass's and the gather's
-# from profiles/ncu_full_gather_x2_triclinic1m.md, the z/y passes' from
-# profiles/dram_per_kernel_water_triclinic_fft_gather.md; the water box's from
-# profiles/dram_per_kernel_water.md.  None: not captured for the current
+# that stay in the 126 MB L2 past the kernel's end are not counted.  The figures
+# at 256^3 are from profiles/launches_triclinic1m.md; the water box's from
+# profiles/dram_per_kernel_water.md (of the kernels before the current z passes
+# and sort).  None: not captured for the current
 # kernels.
 NCU_TRAFFIC = {
     "water": {"cell_sort": 7.48e6, "spread": 2.33e6, "fft_forward": 7.30e6, "convolution": 28.99e6,
               "fft_inverse": 7.38e6, "gather": 6.70e6},
-    "triclinic": {"cell_sort": 119.30e6, "spread": 44.54e6, "fft_forward": 163.58e6, "convolution": 162.71e6,
-                  "fft_inverse": 165.67e6, "gather": 160.72e6},
+    "triclinic": {"cell_sort": 119.20e6, "spread": 38.12e6, "fft_forward": 159.62e6, "convolution": 159.49e6,
+                  "fft_inverse": 167.76e6, "gather": 156.96e6},
 }
 # Kernels of each stage (the roofline is reported for the longest stage that
 # is a single kernel launch).
