@@ -61,8 +61,14 @@
 namespace spme {
 
 constexpr int kRealWords = 16;  // per-group partials: e, W[6], q^2, q, pad
-constexpr int kRealWarps = 4;   // warps per block of the pair kernel
-constexpr int kRealBlocksPerSM = 6;
+// Warps per block of the pair kernel and blocks per SM: 24 warps per SM, the
+// best count of those tried.  The warps take groups independently and share
+// only the table.  98,304-atom water, whole term: 2 warps x 12 blocks 641 us;
+// 4 warps x 5, 6, 7, 8 blocks 658, 649, 652, 682.  Uniform charges (100/nm^3,
+// cutoff 0.9 nm), 2 x 12 against 4 x 6: 98,304 502 against 505 us; 500 to
+// 50,000 and 200,000 charges the same within 1%.
+constexpr int kRealWarps = 2;
+constexpr int kRealBlocksPerSM = 12;
 constexpr int kRealStage = 64;  // candidates staged per round of the walk
 
 // Cubic-Hermite table of erfcx(x) = exp(x^2) erfc(x) on [0, xmax]: interval
