@@ -73,7 +73,7 @@ class SpmePlan:
         if not np.array_equal(L, self.L):
             self.sf._libsfac.set_L(self.sf._data, L.copy())
             self.sf.set_ewald(self.beta, self.max_m)  # influence function of the new box
-            self.L = L.copy()
+            self.L[:] = L  # in place: a batch reads its plans' boxes through this array
 
     def launch(self, x, q, ready):
         """Copies the inputs in and enqueues the solve on the plan's stream
@@ -155,7 +155,11 @@ class SpmeBatch:
                                                     self.dEdL[i])))
             self.sysid = torch.repeat_interleave(torch.arange(B, device=self.device),
                                                  torch.tensor(counts, device=self.device))
+            # the plans' current boxes: every plan keeps its own in a row of this
+            # array, so that there is one record of it whoever sets it
             self.boxes = np.stack([p.L for p in self.plans]) if B else np.zeros((0, 6))
+            for p, row in zip(self.plans, self.boxes):
+                p.L = row
             self._n = np.asarray(counts, dtype=np.int32)
             self._handles = (c_void_p * max(B, 1))(*[p.sf._data for p in self.plans])
             self._lib = _lib()
@@ -166,7 +170,6 @@ class SpmeBatch:
         """The boxes (B, 6) of the next solve; unchanged ones cost nothing."""
         for i in np.nonzero((boxes != self.boxes).any(axis=1))[0]:
             self.plans[i].set_box(boxes[i])
-            self.boxes[i] = boxes[i]
 
     def solve(self, x, q, stream):
         """Enqueues all systems' solves after `stream`'s work, on the plans' own

@@ -1,0 +1,35 @@
+"""SpmeBatch calls: boxes changed through a plan."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(40, (24, 24, 24), 4), (60, (24, 25, 27), 6)]
+L0 = np.array([[2.5, 2.4, 2.6, 0.2, -0.1, 0.3], [2.2, 2.3, 2.6, 0.0, 0.1, -0.3]])
+
+
+def _inputs():
+    import torch
+
+    rng = np.random.default_rng(5)
+    N = sum(s[0] for s in SHAPES)
+    return (torch.tensor(rng.uniform(0, 2.2, size=(N, 3)), device="cuda"),
+            torch.tensor(rng.normal(size=N), device="cuda"))
+
+
+def test_box_set_through_a_plan(libsfac_path):
+    """A plan's box set between two calls of its batch is not taken for the
+    box of the calls: every call solves in the boxes that it is given."""
+    import torch
+
+    from ewaldcorrel_b200.autograd import SpmeBatch
+
+    batch = SpmeBatch(SHAPES)
+    x, q = _inputs()
+    L1 = 1.1 * L0
+    want0, want1 = batch(x, q, torch.tensor(L0)).clone(), batch(x, q, torch.tensor(L1)).clone()
+    assert not torch.equal(want0, want1)
+    batch.plans[0].set_box(L0[0])
+    assert torch.equal(batch(x, q, torch.tensor(L1)), want1)
+    batch.plans[1].set_box(L0[1])
+    assert torch.equal(batch(x, q, torch.tensor(L0)), want0)
