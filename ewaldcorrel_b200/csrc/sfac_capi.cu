@@ -91,6 +91,7 @@ struct Handle {
   double *d_x = nullptr, *d_w = nullptr;  // d_w: the last quarter of d_x's allocation
   uint32_t *d_words = nullptr;            // the sort's word buffers, back to back
   SortBuffers sb{};
+  bool counts_clean = false;  // sb's count words are zero, as every sort of the handle wants them on entry
   int gcap = 0;
   double *d_gx = nullptr, *d_gw = nullptr, *d_gout = nullptr;
   int ccap = 0;
@@ -384,6 +385,32 @@ void destroy(Handle *h) {
 
 bool sync(Handle *h) { return CK(h, cudaStreamSynchronize(h->stream)); }
 
+// Zeroes the sort's count words unless the last call that sorted left them so.
+// Each call's own kernels do that; after a call whose later launches failed the
+// words hold offsets, and a sort that began from them would place atoms far
+// past its buffers.
+bool clean_counts(Handle *h) {
+  if (h->counts_clean) return true;
+  const ZeroWords c = sort_count_words(h->geom, -1, h->sb, kSpreadZShift);
+  h->counts_clean = CK(h, cudaMemsetAsync(c.p, 0, sizeof(uint32_t) * c.n, h->stream));
+  return h->counts_clean;
+}
+
+// Before and after the launches of a call that sorts: the words must be zero
+// to begin with, and count as zero again only if every launch succeeded.  After
+// a failure they are zeroed at once (also for graphs that a caller captured
+// earlier), or else before the next call.
+bool begin_sort(Handle *h) {
+  if (!clean_counts(h)) return false;
+  h->counts_clean = false;
+  return true;
+}
+bool end_sort(Handle *h, bool ok) {
+  if (ok) h->counts_clean = true;
+  else clean_counts(h);
+  return ok;
+}
+
 }  // namespace
 
 extern "C" {
@@ -466,8 +493,7 @@ void *sfac_ctor(double L[6], int K[3], int order) {
       n += fft_make_len(h->fft.len[d], K[d], h->d_tw[d], h->stream);
       n += launch_bspline_moduli(K[d], order, h->nodes, h->d_iB[d], h->stream);
     }
-    const ZeroWords counts = sort_count_words(g, -1, h->sb, kSpreadZShift);
-    ok = launched(h, n, "ctor kernels") && CK(h, cudaMemsetAsync(counts.p, 0, sizeof(uint32_t) * counts.n, h->stream)) &&
+    ok = launched(h, n, "ctor kernels") && clean_counts(h) &&
          CK(h, cudaMemsetAsync(h->d_real, 0, sizeof(float) * h->nreal, h->stream)) &&
          CK(h, cudaMemsetAsync(h->d_cplx, 0, sizeof(float2) * h->nmodes, h->stream)) && sync(h);
   }
@@ -496,13 +522,14 @@ void sfac(void *p, int n, const double *w, const double *x) {
       return;
   }
   CK(h, cudaEventRecord(h->ev_in, h->stream));
+  if (!begin_sort(h)) return;
   int k = launch_cell_sort(h->geom, n, h->d_x, h->d_w, h->sb, h->stream, kSpreadZShift, true);
   k += launch_spread(h->geom, h->spline, h->sb.cell_start, h->sb.keys[h->sb.cur], h->sb.rec_sorted, h->d_real,
                      h->stream);
   DeconvArgs dc{h->d_iB[0], h->d_iB[1], h->d_iB[2], h->ldim};
   k += launch_fft_forward(h->fft, h->geom, h->d_real, h->d_cplx, dc,
                           sort_count_words(h->geom, n, h->sb, kSpreadZShift), h->stream);
-  if (!launched(h, k, "sfac kernels")) return;
+  if (!end_sort(h, launched(h, k, "sfac kernels"))) return;
   // The caller may reuse w and x once this returns: wait for the copies only.
   CK(h, cudaEventSynchronize(h->ev_in));
   h->last_n = n;
@@ -1120,9 +1147,11 @@ static int solve_device(Handle *h, int n, const double *x, const double *w, doub
   if (!ensure_atoms(h, n)) return 2;
   if (dEdL && !ensure_cellp(h, n)) return 2;
   if (timed || !h->use_graph) {
+    if (!begin_sort(h)) return 3;
     const int k = enqueue_solve(h, n, x, w, dx, phi, ev, dEdL, timed);
-    if (!launched(h, k, "solve kernels")) return 3;
+    if (!end_sort(h, launched(h, k, "solve kernels"))) return 3;
   } else {
+    if (!clean_counts(h)) return 3;
     const Handle::Key key{n, x, w, dx, phi, ev, dEdL, h->stream, h->version};
     if (!(h->graph && key == h->gkey)) {
       if (h->graph) {
