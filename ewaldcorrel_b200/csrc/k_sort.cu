@@ -748,12 +748,14 @@ __global__ void __launch_bounds__(kSmallThreads) cell_sort_small_kernel(
 // 5 of 16, about one bucket in 70,000 spills) and while they stay small in
 // L2: a solve of 98k atoms on 96^3 (3.5 MB of slots) took 67.8 us against
 // 70.8, 200k on 128^3 126.6 / 129.1, 400k on 160^3 (16 MB) 230.6 / 238.7, but
-// 600k on 192^3 (28 MB) 308.4 / 303.5 and 1M on 256^3 (67 MB) 549.6 / 543.9.
-constexpr double kSlotsMaxBytes = 1 << 24;
+// 600k on 192^3 (28 MB) 308.4 / 303.5 and 1M on 256^3 (67 MB) 549.6 / 543.9.  More
+// are not allocated (slots_fit).
+constexpr size_t kSlotsMaxBytes = 1 << 24;
+bool slots_fit(int nslot, long nbuckets) { return sizeof(uint2) * nslot * (size_t)nbuckets <= kSlotsMaxBytes; }
+
 static bool use_slots(const Geom &g, int n, const SortBuffers &b, int zshift) {
   const double mean = (double)n * (double)(1 << zshift) / ((double)g.K0 * g.K1 * g.K2);
-  return b.slots && 2.0 * mean + 6.0 <= (double)b.nslot &&
-         8.0 * (double)b.nslot * (double)sort_buckets(g, zshift) <= kSlotsMaxBytes;
+  return b.slots && 2.0 * mean + 6.0 <= (double)b.nslot;
 }
 
 void sort_prepare() {

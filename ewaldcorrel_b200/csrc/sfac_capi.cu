@@ -261,8 +261,9 @@ bool ensure_real(Handle *h, int n, long ncell) {
   // slots for the sort while a cell's mean is small (12 points at water's
   // density and a 1 nm cutoff): 2 mean + 6 of them, a multiple of 4
   const double mean = (double)n / (double)ncell;
-  const bool slots = mean <= 28.0;
-  r.sb.nslot = slots ? ((int)(2.0 * mean) + 6 + 4) / 4 * 4 : 0;
+  const int nslot = mean <= 28.0 ? ((int)(2.0 * mean) + 6 + 4) / 4 * 4 : 0;
+  const bool slots = nslot > 0 && slots_fit(nslot, ncell);
+  r.sb.nslot = slots ? nslot : 0;
   bool ok = true;
   for (int i = 0; i < 2 && ok; i++) ok = dalloc(h, &r.sb.keys[i], cap) && dalloc(h, &r.sb.vals[i], cap);
   ok = ok && dalloc(h, &r.sb.tmp, cap) && dalloc(h, &r.sb.tkeys, cap) && dalloc(h, &r.sb.rec, cap) &&
@@ -307,6 +308,12 @@ bool ensure_atoms(Handle *h, int n) {
   h->cap = (int)cap;
   h->version++;  // buffers moved: cached graphs are stale
   return true;
+}
+
+// Words of the real grid's allocation: its nreal points or the sort's slots on it.
+size_t real_words(long nreal, long nbuckets) {
+  const size_t slot_words = slots_fit(kSpreadSlots, nbuckets) ? 2 * (size_t)kSpreadSlots * nbuckets : 0;
+  return slot_words > (size_t)nreal ? slot_words : (size_t)nreal;
 }
 
 bool ensure_cellp(Handle *h, int n) {
@@ -465,23 +472,24 @@ void *sfac_ctor(double L[6], int K[3], int order) {
             CK(h, cudaEventCreateWithFlags(&h->ev_in, cudaEventDisableTiming));
   h->stream = h->own_stream;
   for (int i = 0; i < 7 && ok; i++) ok = CK(h, cudaEventCreate(&h->ev_stage[i]));
-  // the real grid also serves as the sort's slots (before the spread writes it)
-  const size_t slot_words = 2 * kSpreadSlots * (size_t)sort_buckets(g, kSpreadZShift);
-  ok = ok && dalloc(h, &h->d_real, slot_words > (size_t)h->nreal ? slot_words : (size_t)h->nreal) &&
+  // the real grid also serves as the sort's slots, where it takes them (before the spread writes it)
+  const long nbuckets = sort_buckets(g, kSpreadZShift);
+  const bool slots = slots_fit(kSpreadSlots, nbuckets);
+  ok = ok && dalloc(h, &h->d_real, real_words(h->nreal, nbuckets)) &&
        dalloc(h, &h->d_cplx, h->nmodes) &&
        dalloc(h, &h->d_partials,
               (size_t)(fft_x_blocks_max(K[1], K[2]) > kConvBlocks ? fft_x_blocks_max(K[1], K[2]) : kConvBlocks) *
                   kRedWords) &&
        dalloc(h, &h->d_red, kRedWords) && dalloc(h, &h->d_ev, kRedWords) && dalloc(h, &h->d_cell, 1) &&
        dalloc(h, &h->d_ic, 1) &&
-       dalloc(h, &h->sb.cell_start, cell_count_words(sort_buckets(g, kSpreadZShift), true));
+       dalloc(h, &h->sb.cell_start, cell_count_words(nbuckets, slots));
   for (int d = 0; d < 3 && ok; d++) ok = dalloc(h, &h->d_iB[d], K[d]) && dalloc(h, &h->d_tw[d], K[d]);
   const size_t hf = (size_t)(2 * h->nmodes > h->nreal ? 2 * h->nmodes : h->nreal);
   ok = ok && CK(h, cudaMallocHost((void **)&h->h_S, sizeof(double) * 2 * h->nmodes)) &&
        CK(h, cudaMallocHost((void **)&h->h_f, sizeof(float) * hf)) &&
        CK(h, cudaMallocHost((void **)&h->h_red, sizeof(double) * kRedWords));
-  h->sb.slots = reinterpret_cast<uint2 *>(h->d_real);
-  h->sb.nslot = kSpreadSlots;
+  h->sb.slots = slots ? reinterpret_cast<uint2 *>(h->d_real) : nullptr;
+  h->sb.nslot = slots ? kSpreadSlots : 0;
   if (ok) {
     g.cell = h->d_cell;
     ok = set_cell(h, L);
@@ -1273,7 +1281,9 @@ unsigned long sfac_footprint_bytes(const int K[3], int n) {
   const size_t K0 = K[0], K1 = K[1], K2 = K[2], ldim = K2 / 2 + 1, nn = (size_t)(n > 0 ? n : 1);
   const size_t cap = nn + nn / 2 + 64;
   const long nzb = ((long)K2 + (1L << kSpreadZShift) - 1) >> kSpreadZShift;
-  size_t b = 8 * kSpreadSlots * K0 * K1 * nzb + 8 * K0 * K1 * ldim + 4 * cell_count_words((long)(K0 * K1) * nzb, true);  // grids, buckets
+  const long nbuckets = (long)(K0 * K1) * nzb;
+  size_t b = 4 * real_words((long)(K0 * K1 * K2), nbuckets) + 8 * K0 * K1 * ldim;  // grids
+  b += 4 * cell_count_words(nbuckets, slots_fit(kSpreadSlots, nbuckets));          // buckets
   b += (K0 + K1 + K2) * 16 + sizeof(RowImg) * K0 * K1;                   // moduli, twiddles, rows
   b += 8 * (size_t)fft_x_blocks_max(K[1], K[2]) * kRedWords;               // partials
   b += cap * (24 + 8 + 8 * 4 + 16 + 16);                                   // sort buffers, records

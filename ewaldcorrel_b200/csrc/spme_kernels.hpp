@@ -48,6 +48,9 @@ size_t cell_count_words(long nbuckets, bool with_slots);
 // the bucket's own 32 points take on the real grid, which is free until the
 // spread writes it and lends the space.
 constexpr int kSpreadSlots = 16;
+// Whether the sort takes nslot slots for each of nbuckets buckets; buffers
+// whose slots it would not take are made without them.
+bool slots_fit(int nslot, long nbuckets);
 // clean: the count words are zero already (sort_count_words), no memset.
 int launch_cell_sort(const Geom &g, int n, const double *x, const double *w, SortBuffers &b, cudaStream_t st,
                      int zshift, bool clean);
