@@ -251,16 +251,25 @@ long sort_buckets(const Geom &g, int zshift) {
 
 // Word layout of the bucket-count region (zero before every sort: by a memset,
 // or by a kernel that runs after the last use of the previous sort's):
-//   [0, nb + 1)            counts, then offsets
-//   [nb + 1, 2 nb + 1)     head: atoms of each bucket in its first H - 1 cells
-//   [2 nb + 1, 3 nb + 1)   tail: atoms of each bucket in its last H cells
-//   [3 nb + 1, + T)        tile sums
-//   [3 nb + 1 + T, + nb)   spill (with slots): last atom (+ 1) of each bucket past its slots
-// (head and tail: the spread's halo of an interior brick starts H cells
-// before a bucket boundary and ends H - 1 cells after one, H = order / 2.)
-size_t cell_count_words(long nb, bool with_slots) {
-  return (size_t)(3 * nb + 1 + cell_tiles(nb) + (with_slots ? nb : 0));
-}
+//   [0, nb + 1)  counts, then offsets
+//   then nb      head: atoms of each bucket in its first H - 1 cells
+//   then nb      tail: atoms of each bucket in its last H cells
+//   then T       tile sums
+//   then nb      spill (with slots): last atom (+ 1) of each bucket past its slots
+// (head and tail, for buckets of several cells: the spread's halo of an
+// interior brick starts H cells before a bucket boundary and ends H - 1 cells
+// after one, H = order / 2.)
+struct CountWords {
+  long head, tail, tsum, spill, total;
+  CountWords(long nb, int zshift, bool with_slots) {
+    head = nb + 1;
+    tail = head + (zshift > 0 ? nb : 0);
+    tsum = tail + (zshift > 0 ? nb : 0);
+    spill = tsum + cell_tiles(nb);
+    total = spill + (with_slots ? nb : 0);
+  }
+};
+size_t cell_count_words(long nb, int zshift, bool with_slots) { return (size_t)CountWords(nb, zshift, with_slots).total; }
 
 // Bucket of a cell key (see above).
 struct BucketMap {
@@ -770,7 +779,7 @@ void sort_prepare() {
 ZeroWords sort_count_words(const Geom &g, int n, const SortBuffers &b, int zshift) {
   const long nb = sort_buckets(g, zshift);
   return ZeroWords{reinterpret_cast<uint32_t *>(b.cell_start),
-                   (long)cell_count_words(nb, n < 0 ? b.slots != nullptr : use_slots(g, n, b, zshift))};
+                   CountWords(nb, zshift, n < 0 ? b.slots != nullptr : use_slots(g, n, b, zshift)).total};
 }
 
 int launch_cell_sort(const Geom &g, int n, const double *x, const double *w, SortBuffers &b, cudaStream_t st,
@@ -780,8 +789,9 @@ int launch_cell_sort(const Geom &g, int n, const double *x, const double *w, Sor
   const int tshift = cell_tile_shift(nb);
   const BucketMap bm = bucket_map(g, zshift);
   uint32_t *count = reinterpret_cast<uint32_t *>(b.cell_start);
-  uint32_t *head = count + (nb + 1), *tail = count + (2 * nb + 1);
-  uint32_t *tsum = count + (3 * nb + 1), *spill = tsum + ntiles;
+  const bool slots = use_slots(g, n, b, zshift);
+  const CountWords cw(nb, zshift, slots);
+  uint32_t *head = count + cw.head, *tail = count + cw.tail, *tsum = count + cw.tsum, *spill = count + cw.spill;
   const int ht_h = zshift > 0 ? g.order / 2 : 0;  // head/tail counts for the spread's buckets only
   b.cur = 0;
   if (n <= kSmallAtoms && nb <= kSmallBuckets) {
@@ -789,11 +799,10 @@ int launch_cell_sort(const Geom &g, int n, const double *x, const double *w, Sor
         g, n, x, w, bm, ht_h, b.cell_start, head, tail, b.tkeys, b.tmp, b.keys[0], b.vals[0], b.rec, b.rec_sorted);
     return 1;
   }
-  const bool slots = use_slots(g, n, b, zshift);
   // tile sums taken while counting, while they are few (more: one pass over the counts)
   const bool count_tiles = ntiles > 1 && ntiles <= kCountTiles && n > 0;
   const Slots sl{slots ? b.slots : nullptr, b.nslot, spill, b.next, (uint32_t)nb};
-  if (!clean) cudaMemsetAsync(count, 0, sizeof(uint32_t) * cell_count_words(nb, slots), st);
+  if (!clean) cudaMemsetAsync(count, 0, sizeof(uint32_t) * cw.total, st);
   int launches = 0;
   if (n > 0) {
     key_count_kernel<<<ceil_div(n, 256), 256, 0, st>>>(g, n, x, w, b.keys[1], b.vals[1], b.rec, count, bm,

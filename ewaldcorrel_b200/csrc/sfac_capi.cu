@@ -268,7 +268,7 @@ bool ensure_real(Handle *h, int n, long ncell) {
   for (int i = 0; i < 2 && ok; i++) ok = dalloc(h, &r.sb.keys[i], cap) && dalloc(h, &r.sb.vals[i], cap);
   ok = ok && dalloc(h, &r.sb.tmp, cap) && dalloc(h, &r.sb.tkeys, cap) && dalloc(h, &r.sb.rec, cap) &&
        dalloc(h, &r.sb.rec_sorted, cap) &&
-       dalloc(h, &r.sb.hist, cap) && dalloc(h, &r.sb.cell_start, cell_count_words(ncell, slots)) &&
+       dalloc(h, &r.sb.hist, cap) && dalloc(h, &r.sb.cell_start, cell_count_words(ncell, 0, slots)) &&
        (!slots || (dalloc(h, &r.sb.slots, (size_t)r.sb.nslot * ncell) && dalloc(h, &r.sb.next, cap))) &&
        dalloc(h, &r.rec, cap) && dalloc(h, &r.x, 3 * (size_t)cap) && dalloc(h, &r.w, cap) &&
        dalloc(h, &r.dx, 3 * (size_t)cap) && dalloc(h, &r.part, real_partial_words(cap)) && dalloc(h, &r.out, 16) &&
@@ -482,7 +482,7 @@ void *sfac_ctor(double L[6], int K[3], int order) {
                   kRedWords) &&
        dalloc(h, &h->d_red, kRedWords) && dalloc(h, &h->d_ev, kRedWords) && dalloc(h, &h->d_cell, 1) &&
        dalloc(h, &h->d_ic, 1) &&
-       dalloc(h, &h->sb.cell_start, cell_count_words(nbuckets, slots));
+       dalloc(h, &h->sb.cell_start, cell_count_words(nbuckets, kSpreadZShift, slots));
   for (int d = 0; d < 3 && ok; d++) ok = dalloc(h, &h->d_iB[d], K[d]) && dalloc(h, &h->d_tw[d], K[d]);
   const size_t hf = (size_t)(2 * h->nmodes > h->nreal ? 2 * h->nmodes : h->nreal);
   ok = ok && CK(h, cudaMallocHost((void **)&h->h_S, sizeof(double) * 2 * h->nmodes)) &&
@@ -1283,7 +1283,7 @@ unsigned long sfac_footprint_bytes(const int K[3], int n) {
   const long nzb = ((long)K2 + (1L << kSpreadZShift) - 1) >> kSpreadZShift;
   const long nbuckets = (long)(K0 * K1) * nzb;
   size_t b = 4 * real_words((long)(K0 * K1 * K2), nbuckets) + 8 * K0 * K1 * ldim;  // grids
-  b += 4 * cell_count_words(nbuckets, slots_fit(kSpreadSlots, nbuckets));          // buckets
+  b += 4 * cell_count_words(nbuckets, kSpreadZShift, slots_fit(kSpreadSlots, nbuckets));  // buckets
   b += (K0 + K1 + K2) * 16 + sizeof(RowImg) * K0 * K1;                   // moduli, twiddles, rows
   b += 8 * (size_t)fft_x_blocks_max(K[1], K[2]) * kRedWords;               // partials
   b += cap * (24 + 8 + 8 * 4 + 16 + 16);                                   // sort buffers, records

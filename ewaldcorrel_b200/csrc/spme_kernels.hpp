@@ -33,7 +33,7 @@ struct SortBuffers {
   float4 *rec;         // (frac0, frac1, frac2, charge) in input order (cap)
   float4 *rec_sorted;  // the same in cell order (cap)
   uint32_t *hist;      // arrival counters of the buckets too large for ranking in place (cap)
-  int *cell_start;     // cell_count_words(nb): nb + 1 bucket counts -> offsets, then the other words
+  int *cell_start;     // cell_count_words(): nb + 1 bucket counts -> offsets, then the other words
   uint2 *slots;        // nslot (a multiple of 4) x buckets scratch of the sort by slots; null: not used
   uint32_t *next;      // chain of the atoms past their bucket's slots (cap; with slots)
   int nslot;
@@ -43,7 +43,7 @@ struct SortBuffers {
 // The spread's bucket: 32 z cells (its bricks are 32 points deep in z).
 constexpr int kSpreadZShift = 5;
 long sort_buckets(const Geom &g, int zshift);
-size_t cell_count_words(long nbuckets, bool with_slots);
+size_t cell_count_words(long nbuckets, int zshift, bool with_slots);
 // Slots per bucket of the spread's sort: 16 of 8 bytes are the 128 bytes that
 // the bucket's own 32 points take on the real grid, which is free until the
 // spread writes it and lends the space.

@@ -55,10 +55,20 @@ def test_device_memory_without_slots(libsfac_path):
     used, s = _device_bytes(lambda: E.Sfac(L, K, 4))
     assert used < _footprint(s._libsfac, K, 1)
     del s
-    # a fine coarse grid: 2.1M cells or more, from 134 MB of slots, 25 MB of counts
-    def real():
-        warm.real_space(q, x, 3.0, 2.0 * 10.0 / 128)
-        return None
-
-    used, _ = _device_bytes(real)
+    # a fine coarse grid: 2.1M cells, 134 MB of slots, 25 MB of counts
+    used, _ = _device_bytes(lambda: warm.real_space(q, x, 3.0, 2.0 * 10.0 / 128))
     assert used < 64 * MB
+
+
+@pytest.mark.gpu
+def test_real_space_count_words(libsfac_path):
+    """The real-space sort keeps, and zeroes on every call, one count word per
+    coarse cell: 16.8M cells here, 67 MB; head and tail counts are the spread's."""
+    from ewaldcorrel_b200 import ewald as E
+
+    L = np.array([10.0, 10.0, 10.0, 0, 0, 0])
+    s = E.Sfac(L, np.array([16, 16, 16]), 4)
+    x, q = np.random.default_rng(0).uniform(0, 10, size=(500, 3)), np.ones(500)
+    s.real_space(q, x, 3.0, 1.0)
+    used, _ = _device_bytes(lambda: s.real_space(q, x, 3.0, 2.0 * 10.0 / 256))
+    assert used < 2 * 4 * 256**3
