@@ -111,9 +111,10 @@ struct Handle {
     SortBuffers sb{};
     int cap = 0;
     long ncell = 0;
-    double4 *rec = nullptr;
-    double *x = nullptr, *w = nullptr, *dx = nullptr, *part = nullptr, *out = nullptr;
-    float4 *tab = nullptr;  // erfcx table of the pair kernel
+    uint32_t *words = nullptr;  // the sort's word buffers, back to back
+    double4 *rec = nullptr;     // then the sort's two record buffers and tab
+    double *x = nullptr, *w = nullptr, *dx = nullptr, *part = nullptr, *out = nullptr;  // one allocation, at x
+    float4 *tab = nullptr;      // erfcx table of the pair kernel
   } rs;
   // pipelined de2 / potl: copy-in and copy-out streams, per-chunk events
   cudaStream_t s_in = nullptr, s_out = nullptr;
@@ -229,34 +230,21 @@ void make_spline(int n, Spline &S, SplineNodes &nodes) {
 
 void free_real(Handle *h) {
   Handle::RealBufs &r = h->rs;
-  for (int i = 0; i < 2; i++) {
-    dfree(r.sb.keys[i]);
-    dfree(r.sb.vals[i]);
-  }
-  dfree(r.sb.tmp);
-  dfree(r.sb.tkeys);
-  dfree(r.sb.next);
-  dfree(r.sb.slots);
-  dfree(r.sb.rec);
-  dfree(r.sb.rec_sorted);
-  dfree(r.sb.hist);
-  dfree(r.sb.cell_start);
+  dfree(r.words);
   dfree(r.rec);
   dfree(r.x);
-  dfree(r.w);
-  dfree(r.dx);
-  dfree(r.part);
-  dfree(r.out);
-  dfree(r.tab);
+  dfree(r.sb.cell_start);
+  dfree(r.sb.slots);
   r.cap = 0;
   r.ncell = 0;
 }
 
-// Buffers of the real-space term for n points on a coarse grid of ncell cells.
+// Buffers of the real-space term for n points on a coarse grid of ncell cells,
+// in five allocations (a call that needs new buffers waits for each of them).
 bool ensure_real(Handle *h, int n, long ncell) {
   Handle::RealBufs &r = h->rs;
-  if (n <= r.cap && ncell == r.ncell && r.out) return true;
-  const int cap = n > r.cap ? n + n / 2 + 64 : r.cap;
+  if (n <= r.cap && ncell == r.ncell && r.x) return true;
+  const size_t cap = n > r.cap ? ((size_t)n + n / 2 + 64 + 3) / 4 * 4 : r.cap;
   free_real(h);
   // slots for the sort while a cell's mean is small (12 points at water's
   // density and a 1 nm cutoff): 2 mean + 6 of them, a multiple of 4
@@ -264,20 +252,24 @@ bool ensure_real(Handle *h, int n, long ncell) {
   const int nslot = mean <= 28.0 ? ((int)(2.0 * mean) + 6 + 4) / 4 * 4 : 0;
   const bool slots = nslot > 0 && slots_fit(nslot, ncell);
   r.sb.nslot = slots ? nslot : 0;
-  bool ok = true;
-  for (int i = 0; i < 2 && ok; i++) ok = dalloc(h, &r.sb.keys[i], cap) && dalloc(h, &r.sb.vals[i], cap);
-  ok = ok && dalloc(h, &r.sb.tmp, cap) && dalloc(h, &r.sb.tkeys, cap) && dalloc(h, &r.sb.rec, cap) &&
-       dalloc(h, &r.sb.rec_sorted, cap) &&
-       dalloc(h, &r.sb.hist, cap) && dalloc(h, &r.sb.cell_start, cell_count_words(ncell, 0, slots)) &&
-       (!slots || (dalloc(h, &r.sb.slots, (size_t)r.sb.nslot * ncell) && dalloc(h, &r.sb.next, cap))) &&
-       dalloc(h, &r.rec, cap) && dalloc(h, &r.x, 3 * (size_t)cap) && dalloc(h, &r.w, cap) &&
-       dalloc(h, &r.dx, 3 * (size_t)cap) && dalloc(h, &r.part, real_partial_words(cap)) && dalloc(h, &r.out, 16) &&
-       dalloc(h, &r.tab, kRealTab);
-  if (!ok) {
+  const size_t part = real_partial_words((int)cap);
+  if (!(dalloc(h, &r.words, (slots ? 8 : 7) * cap) && dalloc(h, &r.rec, 2 * cap + kRealTab / 2) &&
+        dalloc(h, &r.x, 7 * cap + part + 16) && dalloc(h, &r.sb.cell_start, cell_count_words(ncell, 0, slots)) &&
+        (!slots || dalloc(h, &r.sb.slots, (size_t)r.sb.nslot * ncell)))) {
     free_real(h);
     return false;
   }
-  r.cap = cap;
+  uint32_t **words[8] = {&r.sb.keys[0], &r.sb.keys[1], &r.sb.vals[0], &r.sb.vals[1],
+                         &r.sb.tkeys,   &r.sb.tmp,     &r.sb.hist,    &r.sb.next};
+  for (int i = 0; i < 8; i++) *words[i] = i < 7 || slots ? r.words + i * cap : nullptr;
+  r.sb.rec = reinterpret_cast<float4 *>(r.rec + cap);
+  r.sb.rec_sorted = r.sb.rec + cap;
+  r.tab = r.sb.rec_sorted + cap;
+  r.w = r.x + 3 * cap;
+  r.dx = r.w + cap;
+  r.part = r.dx + 3 * cap;
+  r.out = r.part + part;
+  r.cap = (int)cap;
   r.ncell = ncell;
   return true;
 }
