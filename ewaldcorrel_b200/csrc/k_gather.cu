@@ -643,17 +643,44 @@ static void gather_tile(const TileArgs &A, const Spline &S, cudaStream_t st) {
   else gather_tile_t<8, kTileX, kTileY, kTileThreads>(A, S, st);
 }
 
-// The brick kernel needs enough points to repay its set-up (a dozen dependent
-// steps before the first stencil) and enough taps per point to repay its
-// copy.  Thread per point / bricks, us: order 6, 50k points on 72^3 20.5 / 18.5,
-// 100k on 120^3 26.6 / 25.6, 200k on 120^3 39.8 / 30.7, 400k on 192^3 81 / 55,
-// 1M on 256^3 182 / 135; order 8, 50k on 72^3 28.7 / 30.8, 100k on 120^3
-// 50 / 33, 1M on 256^3 352 / 205; order 4, 100k on 96^3 14.3 / 16.4, 1M on
-// 200^3 77.8 / 79.9 (not taken).  Odd rows are copied value by value: 200k
-// points on 150^3 then took 45.1 us against 45.0 (order 6).
-constexpr int kTileMinPoints = 65536, kTileMinPointsOdd = 262144;
+// Where bricks are the faster gather (sorted points).  A brick copies its halo
+// block and orders its points whatever their number, and one CTA walks through
+// them, kTileThreads at a time: with few points per brick the copy is longer
+// than the points' own loads, with few bricks the SMs have little to overlap,
+// and with many points in few bricks the longest CTA decides.  Evenly filled
+// cubic grids, thread per point / bricks, us (mean: points per 4096 cells):
+//   order 6   70k 256^3 (mean 16) 38.9 / 80.9   260k 256^3 (63) 85.0 / 89.1
+//             195k 200^3 (100) 55.3 / 58.3      274k 224^3 (100) 76.7 / 68.6
+//             105k 120^3 (250) 26.7 / 29.7      110k 144^3 (150) 29.7 / 29.7
+//             150k 160^3 (150) 43.0 / 35.8      520k 256^3 (127) 118.8 / 97.2
+//             1M 256^3 (244) 173.0 / 132.1      1.6M 160^3 (1600) 174.1 / 166.9
+//     384 to 767 bricks: 128k 128^3 (a brick 250) 36.9 / 33.8, 169k 120^3 (352)
+//             36.9 / 31.7, 205k 128^3 (400) 39.9 / 42.1, 512k 128^3 65.6 / 70.7
+//     fewer:  130k 48^3 24.6 / 87.1, 260k 72^3 36.9 / 58.4, 165k 104^3 32.8 / 33.9
+//   order 8   66k 256^3 (16) 63.5 / 97.2        82k 224^3 (30) 69.7 / 74.8
+//             66k 192^3 (38) 56.3 / 52.2        130k 256^3 (32) 140.3 / 103.4
+//             1M 256^3 (244) 347.3 / 207.9      2.1M 176^3 (1600) 405.5 / 357.3
+//     384 to 767 bricks: 512k 128^3 (1000) 122.9 / 105.5, 675k 120^3 (1600) 142.3 /
+//             117.8, 819k 128^3 (1600) 166.0 / 175.1, 1M 128^3 (1953) 190.5 / 179.2
+//     two per SM or fewer: 66k 96^3 (a brick 306) 32.8 / 29.8, 130k 96^3 (602)
+//             51.2 / 42.0, 260k 90^3 (1204) 65.6 / 72.7, 130k 48^3 38.9 / 126.0
+//     between: 69k 104^3 (189) 34.8 / 37.9, 274k 104^3 (754) 72.7 / 78.8
+// Odd rows are copied value by value and need twice the points: order 6, 271k
+// 195^3 (150) 70.6 / 72.7, 327k 175^3 (250) 66.5 / 62.5; order 8, 109k 195^3 (60)
+// 75.8 / 85.0, 262k 225^3 (94) 163.8 / 132.1.  Order 4: 100k on 96^3 14.3 / 16.4, 1M
+// on 200^3 77.8 / 79.9 (not taken).
+constexpr int kTileCells = kTileX * kTileY * 32;
+constexpr int kTileMinPointsOdd = 262144;
 static bool use_tiles(const Geom &g, int n) {
-  return g.order >= 6 && n >= ((g.K2 & 1) ? kTileMinPointsOdd : kTileMinPoints);
+  if (g.order < 6) return false;
+  const bool p6 = g.order == 6, odd = g.K2 & 1;
+  const double mean = (double)n * kTileCells / ((double)g.K0 * g.K1 * g.K2);
+  const long bricks = (long)((g.K0 + kTileX - 1) / kTileX) * ((g.K1 + kTileY - 1) / kTileY) * ((g.K2 + 31) / 32);
+  const double per = (double)n / (double)bricks;
+  if (n < (odd ? kTileMinPointsOdd : (p6 ? 122880 : 65536))) return false;
+  if (mean < (p6 ? (odd ? 200.0 : 96.0) : (odd ? 90.0 : 31.0)) || mean > (p6 ? 1600.0 : 2000.0)) return false;
+  if (p6) return bricks >= 768 || (bricks >= 384 && per <= 384.0);
+  return bricks >= 384 || (bricks >= 208 && bricks <= 2 * 148 && per <= 640.0);
 }
 
 bool gather_uses_buckets(const Geom &g, int n, bool dx, bool phi) { return n > 0 && (dx || phi) && use_tiles(g, n); }
@@ -676,6 +703,11 @@ constexpr int kGatherThreads = 128;
 // 45.2 / 46.0 (not taken).  Sorted points only: de2 of 24k points in input order
 // took 134 us with 8 lanes against 127, its lanes computing the FP64 origin 8 times.
 constexpr int kSplitMaxPoints = 24576;
+
+int gather_route(const Geom &g, int n) {
+  if (use_tiles(g, n)) return 2;
+  return g.order >= 6 && n <= kSplitMaxPoints ? 1 : 0;
+}
 
 template <int P, bool SORTED>
 static int gather_p(const Geom &g, const Spline &S, int n, const double *x, const double *w, const float *grid,

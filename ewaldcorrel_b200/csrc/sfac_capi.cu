@@ -1342,6 +1342,15 @@ int sfac_debug_fail_alloc(int nth) {
   return 0;
 }
 
+int sfac_debug_gather_route(const int K[3], int order, int n) {
+  Geom g{};
+  g.K0 = K[0];
+  g.K1 = K[1];
+  g.K2 = K[2];
+  g.order = order;
+  return gather_route(g, n);
+}
+
 int sfac_debug_spread(void *p, float *grid) {
   Handle *h = H(p);
   if (!h || h->state != 0) return 1;

@@ -196,6 +196,7 @@ int launch_gather(const Geom &g, const Spline &S, int n, const double *x, const 
                   const float *grid, double *dx, double *phi, cudaStream_t st, const uint32_t *perm = nullptr,
                   const uint32_t *keys = nullptr, const float4 *rec = nullptr, const int *cs = nullptr);
 bool gather_uses_buckets(const Geom &g, int n, bool dx, bool phi);  // whether a launch_gather given cs reads it
+int gather_route(const Geom &g, int n);  // of sorted points: 0 a thread per point, 1 eight lanes per point, 2 bricks
 void gather_prepare();  // sets the brick kernels' shared-memory limits once (before any graph capture)
 // Gather + cell adjoint: dE/dL (6 doubles, device) from dE/dx, the virial in ev
 // and the positions; cellp is scratch of gather_cell_words(n) doubles.

@@ -338,6 +338,9 @@ int sfac_check_enabled(void);
 int sfac_check_take(unsigned long long *word);
 int sfac_check_selftest(void);
 int sfac_debug_spread(void *sfac, float *grid);
+/* The gather that a solve of n atoms takes (no device needed): 0 one thread
+ * per point, 1 eight lanes per point, 2 bricks of the grid in shared memory. */
+int sfac_debug_gather_route(const int K[3], int order, int n);
 
 #ifdef __cplusplus
 }
