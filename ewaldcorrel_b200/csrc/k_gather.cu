@@ -1,12 +1,16 @@
 // K6: force and potential gather (de2, sfac.cpp:409-483; potl,
 // sfac.cpp:497-545).
 //
-// One thread per point, so every output has exactly one writer and the sum
-// order is fixed.  The stencil origin is computed in FP64 exactly as the
+// One thread per point, 8 lanes per point (few points) or a CTA per brick of
+// the grid (many): every output has exactly one writer, and the sum order is
+// fixed and the same in all three.  The stencil origin is computed in FP64 exactly as the
 // reference does (u = scale(x)*K, k1 = ceil(u), k0 = (k1 - order/2) mod K);
 // the B-spline weights and the order^3 sum are FP32, factorised as
 // sum_i wx_i sum_j wy_j sum_k wz_k Q  (one pass gives phi and all three
 // derivatives).  The chain rule through iL and the scaling are FP64.
+#include <algorithm>
+#include <cmath>
+
 #include "reduce.cuh"
 #include "spme_kernels.hpp"
 
@@ -203,6 +207,24 @@ __device__ __forceinline__ PointAt point_at(const Geom &g, int r, int n, const d
   return p;
 }
 
+// Stencil sums of a point by one thread.
+template <int P>
+__device__ __forceinline__ void point_sums(const Geom &g, const Spline &S, const float *__restrict__ grid,
+                                           const PointAt &pt, float &pot, float &gx, float &gy, float &gz) {
+  float wx[P], dwx[P], wy[P], dwy[P], wz[P], dwz[P];
+#pragma unroll
+  for (int i = 0; i < P; i++) {
+    dbspl_eval(S, P, pt.t0, i, wx[i], dwx[i]);
+    dbspl_eval(S, P, pt.t1, i, wy[i], dwy[i]);
+    dbspl_eval(S, P, pt.t2, i, wz[i], dwz[i]);
+  }
+  int iy[P];
+  wrap_run<P>(pt.o1, g.K1, iy);
+  with_planes<P>(grid, g, iy, pt.o2, wy, dwy, wz, dwz, [&](auto &&plane) {
+    stencil_sum<P>(g, pt.o0, wx, dwx, plane, pot, gx, gy, gz);
+  });
+}
+
 // CELL: also the per-block sums of s_i (dE/dr)_j over the block's points
 // (s = iL^T x, unwrapped), written to cellp[block][9] in a fixed order.
 // SORTED: thread r handles point perm[r], with the stencil origin from its
@@ -224,21 +246,9 @@ __global__ void __launch_bounds__(256, CELL ? 2 : 3) gather_kernel(Geom g, Splin
   if (r < n) {
     const CellConst cc = *g.cell;
     const PointAt pt = point_at<P, SORTED>(g, r, n, x, sv);
-    const int a = pt.a, o0 = pt.o0, o1 = pt.o1, o2 = pt.o2;
-    const float t0 = pt.t0, t1 = pt.t1, t2 = pt.t2;
-    float wx[P], dwx[P], wy[P], dwy[P], wz[P], dwz[P];
-#pragma unroll
-    for (int i = 0; i < P; i++) {
-      dbspl_eval(S, P, t0, i, wx[i], dwx[i]);
-      dbspl_eval(S, P, t1, i, wy[i], dwy[i]);
-      dbspl_eval(S, P, t2, i, wz[i], dwz[i]);
-    }
-    int iy[P];
-    wrap_run<P>(o1, g.K1, iy);
+    const int a = pt.a;
     float pot = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
-    with_planes<P>(grid, g, iy, o2, wy, dwy, wz, dwz, [&](auto &&plane) {
-      stencil_sum<P>(g, o0, wx, dwx, plane, pot, gx, gy, gz);
-    });
+    point_sums<P>(g, S, grid, pt, pot, gx, gy, gz);
     if (GRAD) {
       const double f = -w[a] * cc.iV;
       const double G0 = (double)gx * f * g.K0, G1 = (double)gy * f * g.K1, G2 = (double)gz * f * g.K2;
@@ -400,6 +410,7 @@ struct TileArgs {
   double *dx, *phi;
   int n, nty, nzb;
   long nb;
+  const uint32_t *crowd;  // the sort's crowd word
 };
 
 // Enqueues the copies of the brick's tile rows in pieces of V values.
@@ -428,6 +439,7 @@ __global__ void __launch_bounds__(NT, 768 / NT) gather_tile_kernel(TileArgs A, S
   TileSmem<P, TX, TY, NT> &sm = *reinterpret_cast<TileSmem<P, TX, TY, NT> *>(gt_smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const Geom &g = A.g;
+  if (__ldg(A.crowd)) return;  // gather_crowded_kernel takes all points
   const int tz = (int)(blockIdx.x % (unsigned)A.nzb), bxy = (int)(blockIdx.x / (unsigned)A.nzb);
   const int x0 = (bxy / A.nty) * TX, y0 = (bxy % A.nty) * TY, z0 = tz * 32;
   const bool near = g.K0 >= C::RX && g.K1 >= C::RY;
@@ -608,10 +620,40 @@ __global__ void __launch_bounds__(NT, 768 / NT) gather_tile_kernel(TileArgs A, S
   }
 }
 
+// After the bricks: zeroes the count words for the next sort (in place of a
+// memset, so that it costs no launch more), and in a crowded system takes all
+// points, one thread each at a time.
+constexpr int kCrowdThreads = 128, kCrowdPerSM = 6;
+template <int P, bool GRAD, bool POT>
+__global__ void __launch_bounds__(kCrowdThreads, kCrowdPerSM) gather_crowded_kernel(TileArgs A, Spline S, SortedView sv,
+                                                                                    ZeroWords zw) {
+  zero_words(zw);
+  if (!__ldg(A.crowd)) return;
+  const Geom &g = A.g;
+  const int step = gridDim.x * kCrowdThreads;
+  for (long r = (long)blockIdx.x * kCrowdThreads + threadIdx.x; r < A.n; r += step) {
+    const CellConst cc = *g.cell;
+    const PointAt pt = point_at<P, true>(g, (int)r, A.n, nullptr, sv);
+    float pot = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
+    point_sums<P>(g, S, A.grid, pt, pot, gx, gy, gz);
+    const long a = pt.a;
+    if (GRAD) {
+      const double f = -A.w[a] * cc.iV;
+      const double G0 = (double)gx * f * g.K0, G1 = (double)gy * f * g.K1, G2 = (double)gz * f * g.K2;
+      A.dx[3 * a + 0] = cc.iL00 * G0;
+      A.dx[3 * a + 1] = cc.iL10 * G0 + cc.iL11 * G1;
+      A.dx[3 * a + 2] = cc.iL20 * G0 + cc.iL21 * G1 + cc.iL22 * G2;
+    }
+    if (POT) A.phi[a] = (double)pot * cc.iV;
+  }
+}
+
 template <int P, int TX, int TY, int NT, bool GRAD, bool POT>
-static void gather_tile_launch(const TileArgs &A, const Spline &S, cudaStream_t st) {
+static void gather_tile_launch(const TileArgs &A, const Spline &S, const SortedView &sv, const ZeroWords &zw,
+                               cudaStream_t st) {
   const unsigned blocks = (unsigned)(((A.g.K0 + TX - 1) / TX) * (long)A.nty * A.nzb);
   gather_tile_kernel<P, TX, TY, NT, GRAD, POT><<<blocks, NT, sizeof(TileSmem<P, TX, TY, NT>), st>>>(A, S);
+  gather_crowded_kernel<P, GRAD, POT><<<kCrowdPerSM * 148, kCrowdThreads, 0, st>>>(A, S, sv, zw);
 }
 
 template <int P, int TX, int TY, int NT>
@@ -624,11 +666,11 @@ static void gather_tile_attr() {
 }
 
 template <int P, int TX, int TY, int NT>
-static void gather_tile_t(TileArgs A, const Spline &S, cudaStream_t st) {
+static void gather_tile_t(TileArgs A, const Spline &S, const SortedView &sv, const ZeroWords &zw, cudaStream_t st) {
   A.nty = (A.g.K1 + TY - 1) / TY;
-  if (A.dx && A.phi) gather_tile_launch<P, TX, TY, NT, true, true>(A, S, st);
-  else if (A.dx) gather_tile_launch<P, TX, TY, NT, true, false>(A, S, st);
-  else gather_tile_launch<P, TX, TY, NT, false, true>(A, S, st);
+  if (A.dx && A.phi) gather_tile_launch<P, TX, TY, NT, true, true>(A, S, sv, zw, st);
+  else if (A.dx) gather_tile_launch<P, TX, TY, NT, true, false>(A, S, sv, zw, st);
+  else gather_tile_launch<P, TX, TY, NT, false, true>(A, S, sv, zw, st);
 }
 
 // The brick shape: 16 x 8 x 32 cells and 256 threads, 3 CTAs per SM.  A
@@ -638,9 +680,10 @@ static void gather_tile_t(TileArgs A, const Spline &S, cudaStream_t st) {
 // 147 / 145, 16 x 8 with 128 threads 147).
 constexpr int kTileX = 16, kTileY = 8, kTileThreads = 256;
 
-static void gather_tile(const TileArgs &A, const Spline &S, cudaStream_t st) {
-  if (A.g.order == 6) gather_tile_t<6, kTileX, kTileY, kTileThreads>(A, S, st);
-  else gather_tile_t<8, kTileX, kTileY, kTileThreads>(A, S, st);
+static void gather_tile(const TileArgs &A, const Spline &S, const SortedView &sv, const ZeroWords &zw,
+                        cudaStream_t st) {
+  if (A.g.order == 6) gather_tile_t<6, kTileX, kTileY, kTileThreads>(A, S, sv, zw, st);
+  else gather_tile_t<8, kTileX, kTileY, kTileThreads>(A, S, sv, zw, st);
 }
 
 // Where bricks are the faster gather (sorted points).  A brick copies its halo
@@ -681,6 +724,25 @@ static bool use_tiles(const Geom &g, int n) {
   if (mean < (p6 ? (odd ? 200.0 : 96.0) : (odd ? 90.0 : 31.0)) || mean > (p6 ? 1600.0 : 2000.0)) return false;
   if (p6) return bricks >= 768 || (bricks >= 384 && per <= 384.0);
   return bricks >= 384 || (bricks >= 208 && bricks <= 2 * 148 && per <= 640.0);
+}
+
+// A brick's CTA takes its points in series, so in a small droplet or a cluster
+// the fullest brick takes longer than one thread per point does for the whole
+// system.  This is the largest bucket of systems that bricks still serve: the
+// one to expect (at 4.5 sigma) where bricks of a dense region hold 512 points
+// and one more per 400 of the system, or 1.5 times the mean.  Beyond it the
+// solve's gather is one thread per point, decided on the device.  Order 6, cubes
+// of a share of the box, thread per point / bricks / this rule, us: 1M on 256^3,
+// 0.1 of the box 117.8 / 103.3 / 103.4, 0.03 113.7 / 238.6 / 111.6, 0.001 93.2 / 3125 /
+// 101.4; 260k on 192^3, 0.3 50.1 / 50.1 / 48.1, 0.1 44.0 / 60.4 / 44.0; 130k on 128^3,
+// 0.3 31.7 / 35.8 / 35.9, 0.1 28.7 / 66.7 / 27.7.  Order 8, 1M on 256^3, 0.1 191.5 /
+// 173.0 / 171.2, 0.03 179.2 / 451.6 / 209.9.  (In one kernel, bricks for the first
+// points of each bucket and CTAs behind them for the others: 0.3 of 256^3 175.1, 260k
+// in 0.1 of 192^3 56.3; the points of full bricks alone one thread each: 72.7 there.)
+int gather_crowd_most(const Geom &g, int n) {
+  const double mean = (double)n * kTileCells / ((double)g.K0 * g.K1 * g.K2);
+  const double bucket = std::max(512.0 + n / 400.0, 1.5 * mean) / (kTileX * kTileY);
+  return (int)(bucket + 4.5 * std::sqrt(bucket) + 2.0);
 }
 
 bool gather_uses_buckets(const Geom &g, int n, bool dx, bool phi) { return n > 0 && (dx || phi) && use_tiles(g, n); }
@@ -760,13 +822,14 @@ static SortedView make_view(const Geom &g, const uint32_t *perm, const uint32_t 
 
 int launch_gather(const Geom &g, const Spline &S, int n, const double *x, const double *w,
                   const float *grid, double *dx, double *phi, cudaStream_t st, const uint32_t *perm,
-                  const uint32_t *keys, const float4 *rec, const int *cs) {
+                  const uint32_t *keys, const float4 *rec, const int *cs, const uint32_t *crowd,
+                  const ZeroWords &zw) {
   if (n <= 0 || (!dx && !phi)) return 0;
   if (cs && use_tiles(g, n)) {
     gather_tile(TileArgs{g, cs, perm, keys, rec, w, grid, dx, phi, n, 0, (g.K2 + 31) / 32,
-                         sort_buckets(g, kSpreadZShift)},
-                S, st);
-    return 1;
+                         sort_buckets(g, kSpreadZShift), crowd},
+                S, make_view(g, perm, keys, rec), zw, st);
+    return 2;
   }
   if (perm) return gather_any<true>(g, S, n, x, w, grid, dx, phi, nullptr, make_view(g, perm, keys, rec), st);
   return gather_any<false>(g, S, n, x, w, grid, dx, phi, nullptr, SortedView{}, st);

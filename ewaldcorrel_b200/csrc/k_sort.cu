@@ -318,13 +318,14 @@ __global__ void __launch_bounds__(256) key_count_kernel(Geom g, int n, const dou
                                                         uint32_t *__restrict__ count, BucketMap bm,
                                                         uint32_t *__restrict__ head, uint32_t *__restrict__ tail,
                                                         int ht_h, Slots sl, uint32_t *__restrict__ tsum, int tshift,
-                                                        int ntiles) {
+                                                        int ntiles, uint32_t *__restrict__ crowd) {
   __shared__ uint32_t th[kCountTiles];
   if (tsum) {
     if (threadIdx.x < ntiles) th[threadIdx.x] = 0u;
     __syncthreads();
   }
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (crowd && a == 0) *crowd = 0u;
   if (a < n) {
     const CellConst cc = *g.cell;
     float4 r;
@@ -403,15 +404,18 @@ __global__ void __launch_bounds__(kScanThreads) tile_sum_kernel(const uint32_t *
 }
 
 // cs[0 .. nscan): per-bucket counts in, exclusive prefix sums out, one CTA
-// per tile; the tile's base is the sum of the earlier tiles' sums.  DONE (the
-// sort by slots): done[offset of a large bucket] = 0, the counter of its atoms
-// that arrive in the merge sort's buffers.  An instance of its own, since the
-// search for large buckets, even only where a thread's sum allows one, takes
-// the scan of 125M counts from 183 to 209 us (23 more with a test per count).
-template <bool DONE>
+// per tile; the tile's base is the sum of the earlier tiles' sums.  MARK: done
+// (the sort by slots; may be null): done[offset of a large bucket] = 0, the
+// counter of its atoms that arrive in the merge sort's buffers; crowd (may be
+// null): *crowd = 1 where a bucket has more than `most` atoms.  An instance of
+// its own, since the search for such buckets, even only where a thread's sum
+// allows one, takes the scan of 125M counts from 183 to 209 us (23 more with a
+// test per count).
+template <bool MARK>
 __global__ void __launch_bounds__(kScanThreads) cell_offsets_kernel(uint32_t *__restrict__ cs, long nscan,
                                                                     int tshift, const uint32_t *__restrict__ tsum,
-                                                                    uint32_t *__restrict__ done) {
+                                                                    uint32_t *__restrict__ done,
+                                                                    uint32_t *__restrict__ crowd, uint32_t most) {
   constexpr int NW = kScanThreads / 32;
   __shared__ uint32_t wsum[NW];
   __shared__ uint32_t red[NW];
@@ -451,10 +455,12 @@ __global__ void __launch_bounds__(kScanThreads) cell_offsets_kernel(uint32_t *__
       o[k] = e;
       e += a[k];
     }
-    if (DONE && s > (uint32_t)kBigCell) {
+    if (MARK && s > min((uint32_t)kBigCell, most)) {
 #pragma unroll
-      for (int k = 0; k < kScanItems; k++)
-        if (a[k] > (uint32_t)kBigCell) done[o[k]] = 0u;
+      for (int k = 0; k < kScanItems; k++) {
+        if (done && a[k] > (uint32_t)kBigCell) done[o[k]] = 0u;
+        if (crowd && a[k] > most) *crowd = 1u;
+      }
     }
     if (full) {
 #pragma unroll
@@ -790,7 +796,7 @@ ZeroWords sort_count_words(const Geom &g, int n, const SortBuffers &b, int zshif
 }
 
 int launch_cell_sort(const Geom &g, int n, const double *x, const double *w, SortBuffers &b, cudaStream_t st,
-                     int zshift, bool clean) {
+                     int zshift, bool clean, const CrowdWord &crowd) {
   const long nb = sort_buckets(g, zshift);
   const long ntiles = cell_tiles(nb);
   const int tshift = cell_tile_shift(nb);
@@ -814,15 +820,16 @@ int launch_cell_sort(const Geom &g, int n, const double *x, const double *w, Sor
   if (n > 0) {
     key_count_kernel<<<ceil_div(n, 256), 256, 0, st>>>(g, n, x, w, b.keys[1], b.vals[1], b.rec, count, bm,
                                                        ht_h ? head : nullptr, tail, ht_h, sl,
-                                                       count_tiles ? tsum : nullptr, tshift, (int)ntiles);
+                                                       count_tiles ? tsum : nullptr, tshift, (int)ntiles, crowd.word);
     launches++;
   }
   if (ntiles > 1 && !count_tiles) {  // one tile (grids up to about 64^3): its scan starts from 0, no tile sums needed
     tile_sum_kernel<<<(unsigned)ntiles, kScanThreads, 0, st>>>(count, nb + 1, tshift, tsum);
     launches++;
   }
-  if (slots) cell_offsets_kernel<true><<<(unsigned)ntiles, kScanThreads, 0, st>>>(count, nb + 1, tshift, tsum, b.hist);
-  else cell_offsets_kernel<false><<<(unsigned)ntiles, kScanThreads, 0, st>>>(count, nb + 1, tshift, tsum, nullptr);
+  const auto offsets = slots || crowd.word ? cell_offsets_kernel<true> : cell_offsets_kernel<false>;
+  offsets<<<(unsigned)ntiles, kScanThreads, 0, st>>>(count, nb + 1, tshift, tsum, slots ? b.hist : nullptr, crowd.word,
+                                                     crowd.word ? (uint32_t)crowd.most : 0xffffffffu);
   launches++;
   if (n > 0 && slots) {
     cell_place_kernel<<<ceil_div(n, 256), 256, 0, st>>>(n, b.keys[1], b.vals[1], b.rec, b.cell_start, bm, sl, b.tkeys,

@@ -91,6 +91,7 @@ struct Handle {
   double *d_x = nullptr, *d_w = nullptr;  // d_w: the last quarter of d_x's allocation
   uint32_t *d_words = nullptr;            // the sort's word buffers, back to back
   SortBuffers sb{};
+  uint32_t *d_crowd = nullptr;  // the sort's crowd word, behind sb's count words
   bool counts_clean = false;  // sb's count words are zero, as every sort of the handle wants them on entry
   int gcap = 0;
   double *d_gx = nullptr, *d_gw = nullptr, *d_gout = nullptr;
@@ -474,7 +475,8 @@ void *sfac_ctor(double L[6], int K[3], int order) {
                   kRedWords) &&
        dalloc(h, &h->d_red, kRedWords) && dalloc(h, &h->d_ev, kRedWords) && dalloc(h, &h->d_cell, 1) &&
        dalloc(h, &h->d_ic, 1) &&
-       dalloc(h, &h->sb.cell_start, cell_count_words(nbuckets, kSpreadZShift, slots));
+       dalloc(h, &h->sb.cell_start, cell_count_words(nbuckets, kSpreadZShift, slots) + 1);
+  if (ok) h->d_crowd = reinterpret_cast<uint32_t *>(h->sb.cell_start) + cell_count_words(nbuckets, kSpreadZShift, slots);
   for (int d = 0; d < 3 && ok; d++) ok = dalloc(h, &h->d_iB[d], K[d]) && dalloc(h, &h->d_tw[d], K[d]);
   const size_t hf = (size_t)(2 * h->nmodes > h->nreal ? 2 * h->nmodes : h->nreal);
   ok = ok && CK(h, cudaMallocHost((void **)&h->h_S, sizeof(double) * 2 * h->nmodes)) &&
@@ -1090,7 +1092,7 @@ static int enqueue_solve(Handle *h, int n, const double *x, const double *w, dou
   cudaStream_t st = h->stream;
   int k = 0;
   // The sort's count words are zero between calls: the first FFT pass after
-  // the spread zeroes them, or a memset at the end where the gather still
+  // the spread zeroes them, or the gather's last kernel where the gather
   // reads the bucket offsets.  (A memset before the sort was one more
   // dependent graph node at the head of every solve.)
   const ZeroWords counts = sort_count_words(h->geom, n, h->sb, kSpreadZShift);
@@ -1098,7 +1100,8 @@ static int enqueue_solve(Handle *h, int n, const double *x, const double *w, dou
   if (timed) CK(h, cudaEventRecord(h->ev_stage[0], st));
   {
     Nvtx r("spme cell sort");
-    k += launch_cell_sort(h->geom, n, x, w, h->sb, st, kSpreadZShift, true);
+    k += launch_cell_sort(h->geom, n, x, w, h->sb, st, kSpreadZShift, true,
+                          late ? CrowdWord{h->d_crowd, gather_crowd_most(h->geom, n)} : CrowdWord{});
   }
   if (timed) CK(h, cudaEventRecord(h->ev_stage[1], st));
   {
@@ -1131,8 +1134,7 @@ static int enqueue_solve(Handle *h, int n, const double *x, const double *w, dou
                             h->sb.rec_sorted);
   else if (n > 0 && (dx || phi))
     k += launch_gather(h->geom, h->spline, n, x, w, h->d_real, dx, phi, st, perm, skeys, h->sb.rec_sorted,
-                       h->sb.cell_start);
-  if (late) CK(h, cudaMemsetAsync(counts.p, 0, sizeof(uint32_t) * counts.n, st));
+                       h->sb.cell_start, h->d_crowd, counts);
   if (timed) CK(h, cudaEventRecord(h->ev_stage[6], st));
   return k;
 }

@@ -52,8 +52,14 @@ constexpr int kSpreadSlots = 16;
 // whose slots it would not take are made without them.
 bool slots_fit(int nslot, long nbuckets);
 // clean: the count words are zero already (sort_count_words), no memset.
+// crowd.word (may be null; not for the one-CTA sort's few atoms): becomes 1 if
+// a bucket has more than crowd.most atoms, else 0.
+struct CrowdWord {
+  uint32_t *word;
+  int most;
+};
 int launch_cell_sort(const Geom &g, int n, const double *x, const double *w, SortBuffers &b, cudaStream_t st,
-                     int zshift, bool clean);
+                     int zshift, bool clean, const CrowdWord &crowd = CrowdWord{});
 // The words of b that a sort of n atoms leaves to be zeroed (n < 0: all that
 // any sort wants zero on entry).
 ZeroWords sort_count_words(const Geom &g, int n, const SortBuffers &b, int zshift);
@@ -194,8 +200,12 @@ int launch_finish(const double *partials, int nblocks, const CellConst *cell, do
 // launch_cell_sort) -- points are then gathered in cell order.
 int launch_gather(const Geom &g, const Spline &S, int n, const double *x, const double *w,
                   const float *grid, double *dx, double *phi, cudaStream_t st, const uint32_t *perm = nullptr,
-                  const uint32_t *keys = nullptr, const float4 *rec = nullptr, const int *cs = nullptr);
-bool gather_uses_buckets(const Geom &g, int n, bool dx, bool phi);  // whether a launch_gather given cs reads it
+                  const uint32_t *keys = nullptr, const float4 *rec = nullptr, const int *cs = nullptr,
+                  const uint32_t *crowd = nullptr, const ZeroWords &zw = ZeroWords{});
+// Whether a launch_gather given cs (the sort's bucket offsets) reads it; that
+// gather reads the sort's crowd word, for gather_crowd_most(), and zeroes zw.
+bool gather_uses_buckets(const Geom &g, int n, bool dx, bool phi);
+int gather_crowd_most(const Geom &g, int n);
 int gather_route(const Geom &g, int n);  // of sorted points: 0 a thread per point, 1 eight lanes per point, 2 bricks
 void gather_prepare();  // sets the brick kernels' shared-memory limits once (before any graph capture)
 // Gather + cell adjoint: dE/dL (6 doubles, device) from dE/dx, the virial in ev

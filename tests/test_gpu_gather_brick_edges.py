@@ -67,3 +67,60 @@ def test_bricks_against_one_thread_per_point(libsfac_path, K, order, n):
 def test_empty_bricks(libsfac_path):
     n, part = 200000, np.array([1.0, 0.5, 0.7])
     check(both((144, 160, 160), 6, n, lambda rng: part * rng.uniform(0, 1, size=(n, 3))))
+
+
+def _clusters(n, *parts):
+    """Shares of the points (the rest: the whole box) in cubes (share, corner, side) of the box."""
+    def s(rng):
+        u, a = rng.uniform(0, 1, size=(n, 3)), 0
+        for share, corner, side in parts:
+            b = a + int(share * n)
+            u[a:b] = corner + side * u[a:b]
+            a = b
+        return u[rng.permutation(n)]
+
+    return s
+
+
+@pytest.mark.parametrize("K,order,n,parts", [
+    ((144, 160, 160), 6, 200000, [(1.0, 0.45, 0.45)]),            # a droplet in a tenth of the box
+    ((160, 160, 160), 8, 70000, [(1.0, 0.98, 0.1)]),              # across the boundaries
+    ((130, 129, 100), 6, 122880, [(0.5, 0.1, 0.001)]),            # one bucket with half of the points
+    ((200, 129, 101), 8, 262144, [(0.3, 0.5, 0.2), (0.2, 0.1, 0.02)]),
+    ((9, 700, 384), 6, 122880, [(0.9, 0.3, 0.3)]),
+    ((300, 300, 20), 6, 122880, [(0.2, 0.7, 0.05)]),
+    ((160, 160, 160), 6, 1000000, [(0.00003, 0.2, 1e-4)]),        # 30 points more in one of evenly filled buckets
+])
+def test_crowded_buckets(libsfac_path, K, order, n, parts):
+    """Clusters of every size: by bricks or, where the sort finds a bucket
+    above the limit, by one thread per point."""
+    check(both(K, order, n, _clusters(n, *parts)))
+
+
+def test_every_solve_decides_anew(libsfac_path):
+    """Evenly filled and crowded systems in turn on one handle, through its
+    graph: each has the bits of a handle of its own."""
+    import torch
+
+    from ewaldcorrel_b200.device import SpmeSolver
+
+    K, order, n = (160, 160, 160), 6, 150000
+    rng = np.random.default_rng(3)
+    x = torch.empty((n, 3), dtype=torch.float64, device="cuda")
+    q = torch.tensor(rng.normal(size=n), device="cuda")
+    out = [torch.empty_like(x), torch.empty_like(q)]
+    sets = [torch.tensor(side * rng.uniform(0, 1, size=(n, 3)) @ configs.LofS(TRI), device="cuda") for side in (1, 0.1)]
+
+    def solve(s, k):
+        x.copy_(sets[k])
+        torch.cuda.synchronize()
+        s.solve(x, q, *out)
+        torch.cuda.synchronize()
+        return [a.clone() for a in out]
+
+    new = lambda: SpmeSolver(TRI, K, order, 3.2, configs.MAX_M_FACTOR * 3.2)  # noqa: E731
+    want = [solve(new(), k) for k in (0, 1)]
+    one = new()
+    for k in (0, 1, 0, 0, 1, 1, 0):
+        for a, b in zip(solve(one, k), want[k]):
+            assert torch.equal(a, b)
