@@ -177,13 +177,15 @@ class SpmeBatch:
     def solve(self, x, q, stream):
         """Enqueues all systems' solves after `stream`'s work, on the plans' own
         streams, and makes `stream` wait for them: (E, dE/dx, phi, dE/dL), new tensors."""
-        N = self.offsets[-1]
-        # copy_ would broadcast fewer rows over all systems
-        if x.dim() != 2 or x.shape[1] != 3 or q.dim() != 1 or min(x.shape[0], q.shape[0]) < N:
-            raise RuntimeError(f"positions {tuple(x.shape)} and charges {tuple(q.shape)} for {N} charges")
+        if x.shape != self.x.shape or q.shape != self.q.shape:
+            # copy_ would broadcast fewer rows over all systems; rows past the charges are not read
+            N = self.offsets[-1]
+            if x.dim() != 2 or x.shape[1] != 3 or q.dim() != 1 or min(x.shape[0], q.shape[0]) < N:
+                raise RuntimeError(f"positions {tuple(x.shape)} and charges {tuple(q.shape)} for {N} charges")
+            x, q = x[:N], q[:N]
         stream.wait_event(self._free)
-        self.x.copy_(x[:N])
-        self.q.copy_(q[:N])
+        self.x.copy_(x)
+        self.q.copy_(q)
         rc = self._lib.sfac_solve_device_many(len(self.plans), self._handles, self._n.ctypes.data, self.x.data_ptr(),
                                               self.q.data_ptr(), self.dx.data_ptr(), self.phi.data_ptr(),
                                               self.ev.data_ptr(), self.dEdL.data_ptr(), c_void_p(stream.cuda_stream))
