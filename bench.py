@@ -179,15 +179,14 @@ def algorithmic_bytes(n, K):
 # DRAM bytes (read + write) per launch of each stage's kernels, from ncu
 # captures of a plain solve (cold caches; summaries in profiles/).  Writes
 # that stay in the 126 MB L2 past the kernel's end are not counted.  The figures
-# at 256^3 are from profiles/launches_triclinic1m.md; the water box's from
-# profiles/dram_per_kernel_water.md (of the kernels before the current z passes
-# and sort).  None: not captured for the current
+# at 256^3 are from profiles/launches_triclinic1m.md, the water box's from
+# profiles/dram_per_kernel_water.md.  None: not captured for the current
 # kernels.
 NCU_TRAFFIC = {
-    "water": {"cell_sort": 7.48e6, "spread": 2.33e6, "fft_forward": 7.30e6, "convolution": 28.99e6,
+    "water": {"cell_sort": 7.31e6, "spread": 2.33e6, "fft_forward": 7.30e6, "convolution": 28.99e6,
               "fft_inverse": 7.38e6, "gather": 6.70e6},
-    "triclinic": {"cell_sort": 119.20e6, "spread": 38.12e6, "fft_forward": 159.62e6, "convolution": 159.49e6,
-                  "fft_inverse": 167.76e6, "gather": 156.96e6},
+    "triclinic": {"cell_sort": 117.92e6, "spread": 37.72e6, "fft_forward": 160.37e6, "convolution": 159.50e6,
+                  "fft_inverse": 167.70e6, "gather": 156.76e6},
 }
 # Kernels of each stage (the roofline is reported for the longest stage that
 # is a single kernel launch).
@@ -197,9 +196,9 @@ STAGE_KERNELS = {
     "fft_forward": "fft_z2_r2c_kernel + fft_y2_kernel<-1>",
     "convolution": "fft_x2_kernel<XM_FWD_CONV_INV> (x FFT, Ewald convolution, energy/virial, inverse x FFT)",
     "fft_inverse": "fft_y2_kernel<+1> (+ energy/virial reduction) + fft_z2_c2r_kernel",
-    "gather": "gather_tile_kernel or gather_kernel (forces + potentials)",
+    "gather": "gather_tile_kernel + gather_crowded_kernel, gather_split_kernel or gather_kernel (forces + potentials)",
 }
-SINGLE_KERNEL_STAGES = ("spread", "convolution", "gather")
+SINGLE_KERNEL_STAGES = ("spread", "convolution")
 
 
 def volume(L):
